@@ -86,8 +86,9 @@ void gemm(const Tensor& A, const Tensor& B, Tensor& C, int64_t M, int64_t N, int
   const int overlap_prev = g_next_gemm_overlap;
   g_next_gemm_overlap = 0;
   TORCH_CHECK(A.is_cuda() && B.is_cuda() && C.is_cuda(), "gemm operands must be CUDA tensors");
-  TORCH_CHECK(A.scalar_type() == at::kBFloat16 && B.scalar_type() == at::kBFloat16,
-              "gemm operands must be bfloat16");
+  TORCH_CHECK(A.scalar_type() == B.scalar_type() &&
+              (A.scalar_type() == at::kBFloat16 || A.scalar_type() == at::kFloat),
+              "gemm operands must both be bfloat16 or both float32");
   TORCH_CHECK(C.scalar_type() == at::kBFloat16 || C.scalar_type() == at::kFloat,
               "gemm output must be bfloat16 or float32");
   c10::cuda::CUDAGuard guard(A.device());
@@ -101,6 +102,7 @@ void gemm(const Tensor& A, const Tensor& B, Tensor& C, int64_t M, int64_t N, int
   g.b_stride_inner = b_si; g.b_stride_outer = b_so;
   g.c_stride_inner = c_si; g.c_stride_outer = c_so;
   g.alpha = (float)alpha;
+  g.ab_fp32 = A.scalar_type() == at::kFloat;
   g.c_fp32 = C.scalar_type() == at::kFloat;
   g.accumulate = accumulate;
   if (bias.has_value()) {
@@ -118,11 +120,11 @@ void gemm(const Tensor& A, const Tensor& B, Tensor& C, int64_t M, int64_t N, int
   if (aux_in.has_value()) { g.aux_in = aux_in->data_ptr(); g.ld_aux = ld_aux; }
   g.causal_tiles = (int)causal_tiles;
   g.overlap_prev = overlap_prev;
-  // scratch for split-K comes from torch's caching allocator, so it is stream-ordered
+  // scratch (split-K, packed operands) comes from torch's caching allocator: stream-ordered
   Tensor ws;
-  const size_t ws_bytes = lt::gemm_split_k_workspace_bytes(g);
+  const size_t ws_bytes = lt::gemm_workspace_bytes(g);
   if (ws_bytes) {
-    ws = torch::empty({(int64_t)(ws_bytes / 4)}, C.options().dtype(torch::kFloat32));
+    ws = torch::empty({(int64_t)((ws_bytes + 3) / 4)}, C.options().dtype(torch::kFloat32));
     g.workspace = ws.data_ptr();
     g.workspace_bytes = ws_bytes;
   }

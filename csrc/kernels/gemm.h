@@ -39,6 +39,7 @@ struct GemmArgs {
   int64_t a_stride_inner = 0, a_stride_outer = 0;
   int64_t b_stride_inner = 0, b_stride_outer = 0;
   int64_t c_stride_inner = 0, c_stride_outer = 0;
+  int ab_fp32 = 0;       // A and B are fp32 (product through bf16 hi + lo parts, see gemm_direct.cu)
   float alpha = 1.0f;
   int c_fp32 = 0;        // output element type: 0 bf16, 1 fp32
   int accumulate = 0;    // C += result
@@ -54,13 +55,17 @@ struct GemmArgs {
                          // 2: skip tiles strictly below (m0 > n0 + BN - 1)
   int causal_k = 0;      // 1: the k loop of the output tile at row m0 stops at k = m0 + 128
                          //    (A is lower block-triangular in 128-blocks: attention dS / P)
+  // k_seg > 0: both operands hold TWO matrices of k_seg (a multiple of 128) along k, the hi and lo
+  // parts of fp32 values, and K = 3 k_seg runs over hi*hi, hi*lo and lo*hi.
+  int k_seg = 0;
   // n > 0: this product reads nothing that the n kernels launched just before it on `stream`
   // write and writes nothing they touch (n = 1: the weight-gradient GEMM after the
   // input-gradient GEMM of the same layer).  Under programmatic dependent launch it then works
   // in their tail and waits for them only before it exits; everything older is complete by
   // then (see the launch rules in common.cuh).  Without the launch attribute it does nothing.
   int overlap_prev = 0;
-  // Optional scratch for split-K (fp32, device memory valid on `stream`).  When a long-K
+  // Optional scratch (device memory valid on `stream`, gemm_workspace_bytes() of it) for packed
+  // operands, see gemm_direct.cu, and for split-K.  When a long-K
   // product has too few output tiles to fill the chip (weight gradients: K = tokens), K is cut
   // into S slices that run as S batches into workspace[S][M][N], and a second kernel sums the
   // slices in fixed order (deterministic) into C.  Without a workspace no split is made.
@@ -92,12 +97,13 @@ struct GemmGather {
   int done_barrier = 1;                   // wait until every peer has finished copying our shard
 };
 
-// Bytes of workspace with which `args` would use split-K (0: it would not split).
-size_t gemm_split_k_workspace_bytes(const GemmArgs& args);
+// Bytes of workspace that `args` would use (0: none).
+size_t gemm_workspace_bytes(const GemmArgs& args);
 
-// Returns cudaSuccess or the launch error. Uses the tensor-core path whenever the
-// operands satisfy TMA alignment (base 16 B aligned, lda/ldb multiples of 8
-// elements); otherwise a SIMT fallback handles the call.
+// Returns cudaSuccess or the launch error.  Operands that satisfy TMA alignment (bf16, base 16 B
+// aligned, lda/ldb multiples of 8 elements) take the TMA kernels; others are loaded by the
+// direct kernel, or packed into the workspace first where the product is large enough to repay
+// the pass; a SIMT kernel handles the smallest ones.
 cudaError_t gemm_bf16(const GemmArgs& args, cudaStream_t stream);
 
 // True if `args` is eligible for the tcgen05 path.

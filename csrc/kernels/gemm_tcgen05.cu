@@ -18,13 +18,16 @@
 // choose_tile() picks kernel and width from a cost model measured on the part; K may be split
 // into slices that run as batches into an fp32 workspace (choose_split, splitk_reduce_kernel);
 // the pair kernel can also pull remote row shards of B over NVLink while it multiplies the
-// local ones (GemmGather).  A SIMT kernel covers the shapes TMA cannot address.
+// local ones (GemmGather).  choose_route() sends what TMA cannot address through gemm_direct.cu
+// (loaded by the CUDA cores, or packed first) and tiny products through a SIMT kernel.
 //
 // This kernel stands in for the reference's cublasSgemm / cublasSgemmStridedBatched
 // (csrc/cuda/ops/matmul.cu:121-133, 177-187) and for its add_broadcast / gelu_bias
 // kernels (csrc/cuda/ops/arithmetic.cu:478-484, csrc/cuda/ops/fused.cu:26-35), which
 // become epilogue options here.
 #include "gemm.h"
+#include "gemm_direct.h"
+#include "gemm_epilogue.cuh"
 #include "sm100_ptx.cuh"
 #include "common.cuh"
 
@@ -37,6 +40,8 @@
 namespace lt {
 
 using namespace ptx;
+
+std::atomic<uint64_t> g_gemm_launches{0};
 
 namespace {
 
@@ -76,112 +81,11 @@ struct TileCfg {
 
 __device__ int g_gemm_error = 0;
 
-struct KernelParams {
-  int M, N, K;
-  int tiles_m, tiles_n, batch_inner, batch_total;
-  int a_mn, b_mn;
-  void* C;
-  long long ldc, c_stride_inner, c_stride_outer;
-  float alpha;
-  int c_fp32, accumulate;
-  const void* bias;
-  int bias_fp32;
-  int act;
-  const __nv_bfloat16* residual;
-  long long ldr;
-  __nv_bfloat16* aux_out;
-  const __nv_bfloat16* aux_in;
-  long long ld_aux;
-  int causal_tiles;
-  int causal_k;
-  int vec_ok;  // C / residual / aux rows allow 16-byte vector access
-  int vec32_ok;  // ... and 32-byte (256-bit) access (bf16 output, residual, aux)
-  int c32_ok;    // fp32 output rows allow 32-byte access
-  // all-gather of B fused into the kernel (g_world <= 1: off)
-  const uint64_t* g_b_ptrs;
-  const uint64_t* g_signal_ptrs;
-  uint32_t* g_flags;
-  int* g_status;
-  long long g_ldb;
-  int g_rank, g_world, g_rows_per_shard, g_done;
-  uint32_t g_epoch;
-  int late_wait;   // GemmArgs::overlap_prev: wait for the previous kernel before exit, not before work
-};
-
-__device__ __forceinline__ float tanh_fast(float x) {
-  float y;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ float gelu_f(float x) {
-  const float k0 = 0.7978845608f, k1 = 0.044715f;
-  float t = tanh_fast(k0 * (x + k1 * x * x * x));
-  return 0.5f * x * (1.0f + t);
-}
-__device__ __forceinline__ float dgelu_f(float x) {
-  const float k0 = 0.7978845608f, k1 = 0.044715f;
-  float t = tanh_fast(k0 * (x + k1 * x * x * x));
-  return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * k0 * (1.0f + 3.0f * k1 * x * x);
-}
-
-// The same two functions on a pair of values with packed f32x2 arithmetic (one instruction
-// per two elements; the tanh stays one MUFU each).  The epilogue of a K = 768 product is bound
-// by instruction issue, so the vector path uses these.
-//   gelu(x)  = h + h t,                  h = x / 2, t = tanh(x (k0 + k0 k1 x^2))
-//   gelu'(x) = s + s r (1 - s) 2,        s = (1 + t) / 2, r = x (k0 + 3 k0 k1 x^2)
-__device__ __forceinline__ float2 tanh_arg2(float2 x, float2 x2) {
-  const float k0 = 0.7978845608f, k0k1 = 0.7978845608f * 0.044715f;
-  return fmul2(x, ffma2(x2, make_float2(k0k1, k0k1), make_float2(k0, k0)));
-}
-__device__ __forceinline__ float2 gelu2(float2 x) {
-  const float2 u = tanh_arg2(x, fmul2(x, x));
-  const float2 t = make_float2(tanh_fast(u.x), tanh_fast(u.y));
-  const float2 h = fmul2(x, make_float2(0.5f, 0.5f));
-  return ffma2(h, t, h);
-}
-// returns v * gelu'(x)
-__device__ __forceinline__ float2 dgelu_mul2(float2 v, float2 x) {
-  const float k0 = 0.7978845608f, k0k1 = 0.7978845608f * 0.044715f;
-  const float2 x2 = fmul2(x, x);
-  const float2 u = tanh_arg2(x, x2);
-  const float2 t = make_float2(tanh_fast(u.x), tanh_fast(u.y));
-  const float2 s = ffma2(t, make_float2(0.5f, 0.5f), make_float2(0.5f, 0.5f));
-  // r2 = 2 x (k0 + 3 k0 k1 x^2)
-  const float2 r2 = fmul2(x, ffma2(x2, make_float2(6.0f * k0k1, 6.0f * k0k1), make_float2(2.0f * k0, 2.0f * k0)));
-  const float2 z = ffma2(fmul2(r2, s), make_float2(-1.0f, -1.0f), r2);      // r2 (1 - s)
-  return fmul2(v, ffma2(s, z, s));
-}
-
-// Scalar epilogue for one element, shared by the tensor-core tail path and the SIMT
-// fallback kernel.
-__device__ __forceinline__ void epilogue_store_scalar(const KernelParams& p, char* c_base,
-                                                      long long row, int col, float acc) {
-  float v = acc * p.alpha;
-  if (p.bias) {
-    v += p.bias_fp32 ? ((const float*)p.bias)[col]
-                     : __bfloat162float(((const __nv_bfloat16*)p.bias)[col]);
-  }
-  if (p.act == GEMM_ACT_GELU) {
-    if (p.aux_out) p.aux_out[row * p.ldc + col] = __float2bfloat16(v);
-    v = gelu_f(v);
-  } else if (p.act == GEMM_ACT_RELU) {
-    if (p.aux_out) p.aux_out[row * p.ldc + col] = __float2bfloat16(v);
-    v = fmaxf(v, 0.0f);
-  } else if (p.act == GEMM_ACT_DGELU) {
-    v *= dgelu_f(__bfloat162float(p.aux_in[row * p.ld_aux + col]));
-  } else if (p.act == GEMM_ACT_DRELU) {
-    v = __bfloat162float(p.aux_in[row * p.ld_aux + col]) > 0.0f ? v : 0.0f;
-  }
-  if (p.residual) v += __bfloat162float(p.residual[row * p.ldr + col]);
-  if (p.c_fp32) {
-    float* c = (float*)c_base + row * p.ldc + col;
-    if (p.accumulate) v += *c;
-    *c = v;
-  } else {
-    __nv_bfloat16* c = (__nv_bfloat16*)c_base + row * p.ldc + col;
-    if (p.accumulate) v += __bfloat162float(*c);
-    *c = __float2bfloat16(v);
-  }
+// The k blocks of A (in: the block of the product) and B for hi*hi, hi*lo, lo*hi (GemmArgs::k_seg).
+__device__ __forceinline__ void hi_lo_blocks(int seg, int& kA, int& kB) {
+  const int part = kA / seg, k = kA - part * seg;
+  kA = part == 2 ? seg + k : k;
+  kB = part == 1 ? seg + k : k;
 }
 
 __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
@@ -248,6 +152,51 @@ __device__ __forceinline__ void load_bf16x32(const __nv_bfloat16* src, float* v,
   }
 }
 
+// v[i] of lane l becomes v[l] of lane i: exchange the halves that bit s of the indices tells apart,
+// s = 16 ... 1.
+__device__ __forceinline__ void warp_transpose32(float (&v)[32], int lane) {
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    const bool up = lane & s;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      if (i & s) continue;
+      const float give = up ? v[i] : v[i + s];
+      const float got = __shfl_xor_sync(0xffffffffu, give, s);
+      if (up) v[i] = got; else v[i + s] = got;
+    }
+  }
+}
+
+// Store of one 32 x 32 block (a lane per row) whose rows cannot be accessed in vectors: turned
+// over within the warp so that a lane holds a column and each store covers a row (lane-per-row
+// stores touch 32 sectors each: [4095,4095] x [4095,4095] in bf16 took 238 us, now 132).  Out of
+// line and with its few arguments by value: the caller's registers belong to the vector path.
+struct UnalignedBlock {
+  void* c;            // element (row 0, this lane's column)
+  long long ldc;
+  float alpha, bias;
+  int rows, c_fp32;   // rows 0: this lane's column is past the edge
+};
+struct Row32 { uint32_t r[32]; };
+__device__ __noinline__ void store_block_unaligned(UnalignedBlock b, int lane, Row32 q) {
+  float v[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(q.r[i]);
+  warp_transpose32(v, lane);
+  if (b.c_fp32) {
+    float* c = (float*)b.c;
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (i < b.rows) c[i * b.ldc] = v[i] * b.alpha + b.bias;
+  } else {
+    __nv_bfloat16* c = (__nv_bfloat16*)b.c;
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (i < b.rows) c[i * b.ldc] = __float2bfloat16(v[i] * b.alpha + b.bias);
+  }
+}
+
 // Epilogue of one 128 x BN accumulator tile: this warp's 32 rows (TMEM lane quadrant `quad`)
 // and every EPI_SPLIT-th 32-column chunk starting at chunk `half`, read from TMEM address
 // `t_row`, written to C.  (Round robin: BN = 192 gives two of the four warps of a quadrant two
@@ -274,8 +223,8 @@ __device__ __forceinline__ void epilogue_tile(const KernelParams& p, uint32_t t_
     const int col0 = n0 + c0;
     if (col0 >= p.N) break;
     const uint32_t* r = &rr[32 * s];
-    if (!row_ok) continue;
     if (p.vec_ok && col0 + 32 <= p.N) {
+      if (!row_ok) continue;
       float v[32];
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
@@ -393,6 +342,24 @@ __device__ __forceinline__ void epilogue_tile(const KernelParams& p, uint32_t t_
         store_bf16x32(cp, v, p.vec32_ok);
       }
     } else {
+      if (!p.vec_ok && p.act == GEMM_ACT_NONE && !p.residual && !p.accumulate) {
+        const int col = col0 + lane, left = p.M - (m0 + quad * 32);
+        UnalignedBlock b;
+        b.c = c_base + ((long long)(m0 + quad * 32) * p.ldc + col) * (long long)esz;
+        b.ldc = p.ldc;
+        b.alpha = p.alpha;
+        b.c_fp32 = p.c_fp32;
+        b.rows = col < p.N ? (left < 32 ? left : 32) : 0;
+        b.bias = b.rows <= 0 || !p.bias ? 0.0f
+                 : p.bias_fp32 ? ((const float*)p.bias)[col]
+                               : __bfloat162float(((const __nv_bfloat16*)p.bias)[col]);
+        Row32 q;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) q.r[i] = r[i];
+        store_block_unaligned(b, lane, q);
+        continue;
+      }
+      if (!row_ok) continue;
       // fully unrolled so the accumulator registers are only ever indexed statically
       // (a dynamic index would force the whole batch into local memory)
 #pragma unroll
@@ -408,7 +375,7 @@ __device__ __forceinline__ void epilogue_tile(const KernelParams& p, uint32_t t_
 template <int BN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                    const __grid_constant__ CUtensorMap tmap_b, const KernelParams p) {
+                    const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ KernelParams p) {
   using Cfg = TileCfg<BN>;
   constexpr int STAGES = Cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
@@ -500,7 +467,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           for (int sub = 0; sub < Cfg::KSUB; ++sub) {
             const uint32_t sa = smem_u32(smem_a + stage * Cfg::A_STAGE + sub * A_STAGE_BYTES);
             const uint32_t sb = smem_u32(smem_b + stage * Cfg::B_STAGE_BYTES + sub * Cfg::B_SUB_BYTES);
-            const int k0 = (kb * Cfg::KSUB + sub) * BK;   // past K: the load returns zeros
+            int k0 = (kb * Cfg::KSUB + sub) * BK;   // past K: the load returns zeros
+            int kB = k0;
+            if (p.k_seg) hi_lo_blocks(p.k_seg, k0, kB);
             if (!p.a_mn) {
               tma_load_4d(sa, &tmap_a, fb, k0, m0, bi, bo);
             } else {
@@ -509,11 +478,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
                 tma_load_4d(sa + c * (64 * BK * 2), &tmap_a, fb, m0 + 64 * c, k0, bi, bo);
             }
             if (!p.b_mn) {
-              tma_load_4d(sb, &tmap_b, fb, k0, n0, bi, bo);
+              tma_load_4d(sb, &tmap_b, fb, kB, n0, bi, bo);
             } else {
 #pragma unroll
               for (int c = 0; c < BN / 64; ++c)
-                tma_load_4d(sb + c * (64 * BK * 2), &tmap_b, fb, n0 + 64 * c, k0, bi, bo);
+                tma_load_4d(sb + c * (64 * BK * 2), &tmap_b, fb, n0 + 64 * c, kB, bi, bo);
             }
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -771,7 +740,7 @@ struct PairCfg {
 template <int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                         const __grid_constant__ CUtensorMap tmap_b, const KernelParams p) {
+                         const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ KernelParams p) {
   using Cfg = PairCfg<BN>;
   constexpr int STAGES = Cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
@@ -875,7 +844,9 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
           for (int sub = 0; sub < Cfg::KSUB; ++sub) {
             const uint32_t sa = smem_u32(smem_a + stage * Cfg::A_STAGE + sub * A_STAGE_BYTES);
             const uint32_t sb = smem_u32(smem_b + stage * Cfg::B_STAGE_BYTES + sub * Cfg::B_SUB_BYTES);
-            const int k0 = (kb * Cfg::KSUB + sub) * BK;   // past K: the load returns zeros
+            int k0 = (kb * Cfg::KSUB + sub) * BK;   // past K: the load returns zeros
+            int kB = k0;
+            if (p.k_seg) hi_lo_blocks(p.k_seg, k0, kB);
             if (!p.a_mn) {
               tma_load_4d_pair(sa, &tmap_a, fb, k0, m0, bi, bo);
             } else {
@@ -884,11 +855,11 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
                 tma_load_4d_pair(sa + c * (64 * BK * 2), &tmap_a, fb, m0 + 64 * c, k0, bi, bo);
             }
             if (!p.b_mn) {
-              tma_load_4d_pair(sb, &tmap_b, fb, k0, n0, bi, bo);
+              tma_load_4d_pair(sb, &tmap_b, fb, kB, n0, bi, bo);
             } else {
 #pragma unroll
               for (int c = 0; c < Cfg::B_ROWS / 64; ++c)
-                tma_load_4d_pair(sb + c * (64 * BK * 2), &tmap_b, fb, n0 + 64 * c, k0, bi, bo);
+                tma_load_4d_pair(sb + c * (64 * BK * 2), &tmap_b, fb, n0 + 64 * c, kB, bi, bo);
             }
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -1007,11 +978,16 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
 }
 
 // ------------------------------------------------------------------------------
-// SIMT fallback: any stride / alignment, same epilogue. Only meant for the small or
-// misaligned shapes TMA cannot address (e.g. a [256, 10] classifier head).
+// SIMT kernel: bf16 or fp32 operands of any stride and alignment, fp32 arithmetic, same
+// epilogue.  For products of a few thousand multiplications (the XOR network's), where filling
+// a 128-row tensor-core tile and draining it takes longer than the sums.
 // ------------------------------------------------------------------------------
+__device__ __forceinline__ float to_f32(float v) { return v; }
+__device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
+
+template <typename E>
 __global__ void __launch_bounds__(256)
-gemm_simt_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B,
+gemm_simt_kernel(const E* __restrict__ A, const E* __restrict__ B,
                  long long a_sm, long long a_sk, long long b_sk, long long b_sn,
                  long long a_stride_inner, long long a_stride_outer, long long b_stride_inner,
                  long long b_stride_outer, KernelParams p) {
@@ -1032,12 +1008,12 @@ gemm_simt_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __res
       int kk, mm;
       if (a_sk == 1) { kk = i % KT; mm = i / KT; } else { mm = i % T; kk = i / T; }
       int m = m0 + mm, k = k0 + kk;
-      sa[kk][mm] = (m < p.M && k < p.K) ? __bfloat162float(A[m * a_sm + k * a_sk]) : 0.0f;
+      sa[kk][mm] = (m < p.M && k < p.K) ? to_f32(A[m * a_sm + k * a_sk]) : 0.0f;
       int nn;
       if (b_sk == 1) { kk = i % KT; nn = i / KT; } else { nn = i % T; kk = i / T; }
       int n = n0 + nn;
       k = k0 + kk;
-      sb[kk][nn] = (n < p.N && k < p.K) ? __bfloat162float(B[k * b_sk + n * b_sn]) : 0.0f;
+      sb[kk][nn] = (n < p.N && k < p.K) ? to_f32(B[k * b_sk + n * b_sn]) : 0.0f;
     }
     __syncthreads();
 #pragma unroll 8
@@ -1099,8 +1075,6 @@ bool encode_operand_map(CUtensorMap* map, const void* base, uint64_t inner, uint
   return r == CUDA_SUCCESS;
 }
 
-std::atomic<uint64_t> g_launches{0};
-
 int num_sms() {
   static int n = 0;
   if (!n) {
@@ -1114,7 +1088,9 @@ int num_sms() {
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-KernelParams make_params(const GemmArgs& a) {
+}  // namespace
+
+KernelParams make_gemm_params(const GemmArgs& a) {
   KernelParams p;
   p.M = a.M; p.N = a.N; p.K = a.K;
   p.tiles_m = 0; p.tiles_n = 0;
@@ -1130,6 +1106,7 @@ KernelParams make_params(const GemmArgs& a) {
   p.aux_in = (const __nv_bfloat16*)a.aux_in; p.ld_aux = a.ld_aux;
   p.causal_tiles = a.causal_tiles;
   p.causal_k = a.causal_k;
+  p.k_seg = a.k_seg;
   const int cvec = a.c_fp32 ? 4 : 8;
   bool v = aligned16(a.C) && (a.ldc % cvec == 0) && (a.c_stride_inner % cvec == 0) &&
            (a.c_stride_outer % cvec == 0);
@@ -1159,6 +1136,8 @@ KernelParams make_params(const GemmArgs& a) {
   return p;
 }
 
+namespace {
+
 template <int BN>
 cudaError_t launch_tc(const GemmArgs& a, cudaStream_t stream) {
   using Cfg = TileCfg<BN>;
@@ -1170,23 +1149,24 @@ cudaError_t launch_tc(const GemmArgs& a, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  KernelParams p = make_params(a);
+  KernelParams p = make_gemm_params(a);
   p.tiles_m = (a.M + BM - 1) / BM;
   p.tiles_n = (a.N + BN - 1) / BN;
   CUtensorMap ta, tb;
   const uint64_t nbi = p.batch_inner, nbo = p.batch_total / p.batch_inner;
+  const uint64_t kx = a.k_seg ? 2 * (uint64_t)a.k_seg : (uint64_t)a.K;   // k extent in memory
   bool ok;
   if (!a.a_mn_major)
-    ok = encode_operand_map(&ta, a.A, a.K, a.M, nbi, nbo, a.lda, a.a_stride_inner,
+    ok = encode_operand_map(&ta, a.A, kx, a.M, nbi, nbo, a.lda, a.a_stride_inner,
                             a.a_stride_outer, BK, BM);
   else
-    ok = encode_operand_map(&ta, a.A, a.M, a.K, nbi, nbo, a.lda, a.a_stride_inner,
+    ok = encode_operand_map(&ta, a.A, a.M, kx, nbi, nbo, a.lda, a.a_stride_inner,
                             a.a_stride_outer, 64, BK);
   if (!a.b_mn_major)
-    ok = ok && encode_operand_map(&tb, a.B, a.K, a.N, nbi, nbo, a.ldb, a.b_stride_inner,
+    ok = ok && encode_operand_map(&tb, a.B, kx, a.N, nbi, nbo, a.ldb, a.b_stride_inner,
                                   a.b_stride_outer, BK, BN);
   else
-    ok = ok && encode_operand_map(&tb, a.B, a.N, a.K, nbi, nbo, a.ldb, a.b_stride_inner,
+    ok = ok && encode_operand_map(&tb, a.B, a.N, kx, nbi, nbo, a.ldb, a.b_stride_inner,
                                   a.b_stride_outer, 64, BK);
   if (!ok) return cudaErrorInvalidValue;
   const long long total = (long long)p.tiles_m * p.tiles_n * p.batch_total;
@@ -1196,7 +1176,7 @@ cudaError_t launch_tc(const GemmArgs& a, cudaStream_t stream) {
   cudaError_t le = launch_pdl(gemm_tcgen05_kernel<BN>, dim3(grid), dim3(NUM_THREADS), Cfg::SMEM_BYTES, stream, ta, tb, p);
   late_wait_commit(lw);
   if (le != cudaSuccess) return le;
-  g_launches.fetch_add(1, std::memory_order_relaxed);
+  g_gemm_launches.fetch_add(1, std::memory_order_relaxed);
   return cudaGetLastError();
 }
 
@@ -1221,7 +1201,7 @@ int pair_clusters() {
       cudaGetLastError();
       c = 0;
     }
-    if (getenv("LT_GEMM_DEBUG")) fprintf(stderr, "pair_clusters<%d> = %d\n", BN, c);
+    if (getenv("LT_GEMM_DEBUG") != nullptr) fprintf(stderr, "pair_clusters<%d> = %d\n", BN, c);
     n = c;
   }
   return n;
@@ -1240,23 +1220,24 @@ cudaError_t launch_pair(const GemmArgs& a, cudaStream_t stream) {
   }
   const int clusters = pair_clusters<BN>();
   if (clusters <= 0) return cudaErrorNotSupported;
-  KernelParams p = make_params(a);
+  KernelParams p = make_gemm_params(a);
   p.tiles_m = (a.M + 2 * BM - 1) / (2 * BM);
   p.tiles_n = (a.N + BN - 1) / BN;
   CUtensorMap ta, tb;
   const uint64_t nbi = p.batch_inner, nbo = p.batch_total / p.batch_inner;
+  const uint64_t kx = a.k_seg ? 2 * (uint64_t)a.k_seg : (uint64_t)a.K;   // k extent in memory
   bool ok;
   if (!a.a_mn_major)
-    ok = encode_operand_map(&ta, a.A, a.K, a.M, nbi, nbo, a.lda, a.a_stride_inner,
+    ok = encode_operand_map(&ta, a.A, kx, a.M, nbi, nbo, a.lda, a.a_stride_inner,
                             a.a_stride_outer, BK, BM);
   else
-    ok = encode_operand_map(&ta, a.A, a.M, a.K, nbi, nbo, a.lda, a.a_stride_inner,
+    ok = encode_operand_map(&ta, a.A, a.M, kx, nbi, nbo, a.lda, a.a_stride_inner,
                             a.a_stride_outer, 64, BK);
   if (!a.b_mn_major)
-    ok = ok && encode_operand_map(&tb, a.B, a.K, a.N, nbi, nbo, a.ldb, a.b_stride_inner,
+    ok = ok && encode_operand_map(&tb, a.B, kx, a.N, nbi, nbo, a.ldb, a.b_stride_inner,
                                   a.b_stride_outer, BK, Cfg::B_ROWS);
   else
-    ok = ok && encode_operand_map(&tb, a.B, a.N, a.K, nbi, nbo, a.ldb, a.b_stride_inner,
+    ok = ok && encode_operand_map(&tb, a.B, a.N, kx, nbi, nbo, a.ldb, a.b_stride_inner,
                                   a.b_stride_outer, 64, BK);
   if (!ok) return cudaErrorInvalidValue;
   const long long total = (long long)p.tiles_m * p.tiles_n * p.batch_total;
@@ -1266,7 +1247,7 @@ cudaError_t launch_pair(const GemmArgs& a, cudaStream_t stream) {
   cudaError_t le = launch_pdl(gemm_tcgen05_pair_kernel<BN>, dim3(grid), dim3(NUM_THREADS), Cfg::SMEM_BYTES, stream, ta, tb, p);
   late_wait_commit(lw);
   if (le != cudaSuccess) return le;
-  g_launches.fetch_add(1, std::memory_order_relaxed);
+  g_gemm_launches.fetch_add(1, std::memory_order_relaxed);
   return cudaGetLastError();
 }
 
@@ -1290,22 +1271,27 @@ int forced_bn() {
 }
 
 cudaError_t launch_simt(const GemmArgs& a, cudaStream_t stream) {
-  KernelParams p = make_params(a);
+  KernelParams p = make_gemm_params(a);
   p.vec_ok = 0;
   long long a_sm = a.a_mn_major ? 1 : a.lda, a_sk = a.a_mn_major ? a.lda : 1;
   long long b_sk = a.b_mn_major ? a.ldb : 1, b_sn = a.b_mn_major ? 1 : a.ldb;
   dim3 grid((a.N + 31) / 32, (a.M + 31) / 32, p.batch_total);
-  gemm_simt_kernel<<<grid, 256, 0, stream>>>(
-      (const __nv_bfloat16*)a.A, (const __nv_bfloat16*)a.B, a_sm, a_sk, b_sk, b_sn,
-      a.a_stride_inner, a.a_stride_outer, a.b_stride_inner, a.b_stride_outer, p);
-  g_launches.fetch_add(1, std::memory_order_relaxed);
+  if (a.ab_fp32)
+    gemm_simt_kernel<float><<<grid, 256, 0, stream>>>(
+        (const float*)a.A, (const float*)a.B, a_sm, a_sk, b_sk, b_sn,
+        a.a_stride_inner, a.a_stride_outer, a.b_stride_inner, a.b_stride_outer, p);
+  else
+    gemm_simt_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(
+        (const __nv_bfloat16*)a.A, (const __nv_bfloat16*)a.B, a_sm, a_sk, b_sk, b_sn,
+        a.a_stride_inner, a.a_stride_outer, a.b_stride_inner, a.b_stride_outer, p);
+  g_gemm_launches.fetch_add(1, std::memory_order_relaxed);
   return cudaGetLastError();
 }
 
 }  // namespace
 
 bool gemm_uses_tensor_cores(const GemmArgs& a) {
-  if (a.M <= 0 || a.N <= 0 || a.K <= 0) return false;
+  if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.ab_fp32) return false;
   if (!aligned16(a.A) || !aligned16(a.B)) return false;
   if (a.lda % 8 || a.ldb % 8) return false;
   if (a.a_stride_inner % 8 || a.a_stride_outer % 8 || a.b_stride_inner % 8 ||
@@ -1383,8 +1369,10 @@ int choose_split(const GemmArgs& a, TileChoice* slice_tile) {
   TileChoice whole = choose_tile(a, a.K, batch, a.c_fp32 != 0);
   *slice_tile = whole;
   if (batch != 1 || a.act != GEMM_ACT_NONE || a.residual || a.aux_out || a.aux_in ||
-      a.causal_tiles || a.causal_k || a.K < 2048 || getenv("LT_GEMM_NO_SPLIT"))
+      a.causal_tiles || a.causal_k || a.k_seg || a.K < 2048)
     return 1;
+  static const bool no_split = getenv("LT_GEMM_NO_SPLIT") != nullptr;
+  if (no_split) return 1;
   // LT_GEMM_SPLIT=n forces a split factor (tuning aid): the slice tile still comes from the model
   static int forced_split = -1;
   if (forced_split < 0) {
@@ -1485,7 +1473,6 @@ splitk_reduce_kernel(const float* __restrict__ ws, int splits, long long slice, 
 }
 
 // every output shape can be split; the workspace rows are padded to four floats
-bool split_k_shape_ok(const GemmArgs&) { return true; }
 inline int ws_ld_of(const GemmArgs& a) { return (a.N + 3) & ~3; }
 inline bool reduce_vec_ok(const GemmArgs& a) {
   return a.N % 4 == 0 && a.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(a.C) & 15) == 0;
@@ -1493,8 +1480,40 @@ inline bool reduce_vec_ok(const GemmArgs& a) {
 
 }  // namespace
 
-size_t gemm_split_k_workspace_bytes(const GemmArgs& a) {
-  if (a.M <= 0 || a.N <= 0 || a.K <= 0 || !gemm_uses_tensor_cores(a) || !split_k_shape_ok(a)) return 0;
+namespace {
+
+// What a product whose operands are not TMA-addressable goes through.
+enum Route { ROUTE_SIMT, ROUTE_DIRECT, ROUTE_PACK };
+
+bool gemm_debug() {
+  static const bool on = getenv("LT_GEMM_DEBUG") != nullptr;
+  return on;
+}
+
+// SIMT up to 2^17 multiplications (5.4 us either way at 64 x 64 x 64; beyond, its serial k loop
+// grows by half a microsecond per 32 values).  Packing costs a launch and a pass over the
+// operands, then runs at TMA speed; the direct kernel reads fp32 through L1 for every tile.
+// Measured: fp32 [1021,777] x [777,1333] 22.9 us packed, 27.3 direct; [1000,1000]^2 22.9 and 19.8;
+// [4096,4096]^2 343 and 558.  The tile model is fitted to launches that follow an idle stream and
+// overestimates the packed product, whose prologue overlaps the packing, by about a quarter.
+Route choose_route(const GemmArgs& a, bool have_workspace) {
+  const long long batch = (long long)(a.batch_inner < 1 ? 1 : a.batch_inner) * (a.batch_outer < 1 ? 1 : a.batch_outer);
+  if ((long long)a.M * a.N * a.K <= 1 << 17) return ROUTE_SIMT;
+  if (!have_workspace || batch > 1 || a.causal_tiles || a.causal_k) return ROUTE_DIRECT;
+  const double elems = (double)a.M * a.K + (double)a.K * a.N;
+  const int parts = a.ab_fp32 ? 3 : 1;
+  const double pack = 0.8 * (3.5e-6 + elems * 8.0 / 4.0e12 + choose_tile(a, parts * a.K, 1, a.c_fp32 != 0).cost);
+  const double direct = gemm_direct_cost(a);
+  if (gemm_debug())
+    fprintf(stderr, "gemm %dx%dx%d: packed %.1f us, direct %.1f us\n", a.M, a.N, a.K, pack * 1e6, direct * 1e6);
+  return pack < direct ? ROUTE_PACK : ROUTE_DIRECT;
+}
+
+}  // namespace
+
+size_t gemm_workspace_bytes(const GemmArgs& a) {
+  if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.gather) return 0;
+  if (!gemm_uses_tensor_cores(a)) return choose_route(a, true) == ROUTE_PACK ? gemm_pack_bytes(a) : 0;
   TileChoice t;
   const int s = choose_split(a, &t);
   return s > 1 ? (size_t)s * (size_t)a.M * (size_t)ws_ld_of(a) * sizeof(float) : 0;
@@ -1521,15 +1540,28 @@ cudaError_t gemm_bf16(const GemmArgs& args, cudaStream_t stream) {
     if (t.cost >= 1e29 || !t.pair) return cudaErrorNotSupported;
     return launch_choice(t, a, stream);
   }
-  if (!gemm_uses_tensor_cores(a)) return launch_simt(a, stream);
+  if (!gemm_uses_tensor_cores(a)) {
+    g_prev_reads_workspace = false;
+    const bool ws = a.workspace && a.workspace_bytes >= gemm_pack_bytes(a);
+    switch (choose_route(a, ws)) {
+      case ROUTE_SIMT: return launch_simt(a, stream);
+      case ROUTE_DIRECT: return gemm_direct(a, stream);
+      case ROUTE_PACK: break;
+    }
+    const cudaError_t e = gemm_pack(a, a.workspace, stream);
+    if (e != cudaSuccess) return e;
+    a.workspace = nullptr;
+    a.overlap_prev = 0;
+    return launch_choice(choose_tile(a, a.K, 1, a.c_fp32 != 0), a, stream);
+  }
   TileChoice tile;
   int splits = choose_split(a, &tile);
   const size_t need = (size_t)splits * (size_t)a.M * (size_t)ws_ld_of(a) * sizeof(float);
-  if (splits > 1 && (!a.workspace || a.workspace_bytes < need || !split_k_shape_ok(a))) {
+  if (splits > 1 && (!a.workspace || a.workspace_bytes < need)) {
     splits = 1;
     tile = choose_tile(a, a.K, 1, a.c_fp32 != 0);
   }
-  if (getenv("LT_GEMM_DEBUG"))
+  if (gemm_debug())
     fprintf(stderr, "gemm %dx%dx%d -> %s BN=%d split %d (model %.1f us)\n", a.M, a.N, a.K,
             tile.pair ? "pair" : "single", tile.bn, splits, tile.cost * 1e6);
   if (splits == 1) {
@@ -1566,19 +1598,20 @@ cudaError_t gemm_bf16(const GemmArgs& args, cudaStream_t stream) {
                               ws_ld, a.C, (long long)a.ldc, a.c_fp32, a.accumulate, a.bias,
                               a.bias_fp32, reduce_vec_ok(a) ? 1 : 0);
   if (re != cudaSuccess) return re;
-  g_launches.fetch_add(1, std::memory_order_relaxed);
+  g_gemm_launches.fetch_add(1, std::memory_order_relaxed);
   return cudaGetLastError();
 }
 
 int gemm_last_device_error() {
   int v = 0;
   cudaMemcpyFromSymbol(&v, g_gemm_error, sizeof(int));
-  return v;
+  return v ? v : gemm_direct_last_error();
 }
 void gemm_clear_device_error() {
   int v = 0;
   cudaMemcpyToSymbol(g_gemm_error, &v, sizeof(int));
+  gemm_direct_clear_error();
 }
-uint64_t gemm_launch_count() { return g_launches.load(); }
+uint64_t gemm_launch_count() { return g_gemm_launches.load(); }
 
 }  // namespace lt

@@ -357,7 +357,8 @@ def dropout_backward(dy: torch.Tensor, p: float, ctx) -> torch.Tensor:
 def gemm(a, b, *, a_t=False, b_t=False, out=None, out_dtype=None, alpha=1.0, accumulate=False,
          bias=None, act=0, residual=None, aux_out=None, aux_in=None, n_valid=None, k_valid=None,
          overlap_prev=0):
-    """C = act(alpha * op(a) @ op(b) + bias) + residual on the tensor cores (bf16 operands).
+    """C = act(alpha * op(a) @ op(b) + bias) + residual on the tensor cores (bf16 operands, or
+    fp32 ones as products of their bf16 hi and lo parts).
 
     a: [M, K] (or [K, M] when a_t), b: [K, N] (or [N, K] when b_t); both 2-d with unit inner
     stride (row strides may exceed the logical width).  `n_valid` restricts the logical N when
@@ -391,22 +392,13 @@ def gemm(a, b, *, a_t=False, b_t=False, out=None, out_dtype=None, alpha=1.0, acc
     return out
 
 
-def _matmul_fp32_tc(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
-    """fp32-accurate product on bf16 tensor cores: a = a_hi + a_lo, b = b_hi + b_lo and
-    a @ b ~= a_hi b_hi + a_hi b_lo + a_lo b_hi, evaluated as ONE GEMM over a 3x longer K."""
-    C = ext()
-    a_hi, a_lo = C.split_bf16(a)
-    b_hi, b_lo = C.split_bf16(b)
-    a3 = torch.cat([a_hi, a_hi, a_lo], dim=1)
-    b3 = torch.cat([b_hi, b_lo, b_hi], dim=0)
-    return gemm(a3, b3, out_dtype=torch.float32)
-
-
 def matmul(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     if a.is_cuda:
         if a.dtype == torch.bfloat16:
             return gemm(_k(a), _k(b.to(torch.bfloat16)))
-        return _matmul_fp32_tc(_k(a.float()), _k(b.float())).to(a.dtype)
+        # fp32-accurate: the kernel multiplies bf16 hi and lo parts of both operands
+        out = gemm(_k(a.float()), _k(b.float()), out_dtype=torch.float32)
+        return out if a.dtype == torch.float32 else out.to(a.dtype)
     return a @ b
 
 
@@ -414,17 +406,9 @@ def bmm(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     if a.is_cuda:
         nb, M, K = a.shape
         N = b.shape[2]
-        if a.dtype == torch.bfloat16:
-            a_, b_ = _k(a), _k(b.to(torch.bfloat16))
-            out = torch.empty((nb, M, N), device=a.device, dtype=torch.bfloat16)
-        else:
-            C = ext()
-            a_hi, a_lo = C.split_bf16(_k(a.float()))
-            b_hi, b_lo = C.split_bf16(_k(b.float()))
-            a_ = torch.cat([a_hi, a_hi, a_lo], dim=2)
-            b_ = torch.cat([b_hi, b_lo, b_hi], dim=1)
-            K = 3 * K
-            out = torch.empty((nb, M, N), device=a.device, dtype=torch.float32)
+        dt = torch.bfloat16 if a.dtype == torch.bfloat16 else torch.float32
+        a_, b_ = _k(a.to(dt)), _k(b.to(dt))
+        out = torch.empty((nb, M, N), device=a.device, dtype=dt)
         ext().gemm(a_, b_, out, M, N, K, K, N, N, False, True, nb, 1, M * K, 0, K * N, 0, M * N, 0,
                    1.0, False, None, 0, None, 0, None, None, 0, 0)
         return out.to(a.dtype)

@@ -33,6 +33,7 @@ class Node:
 
 
 enabled = True
+_GEMM_DTYPES = (torch.bfloat16, torch.float32)
 graph: List[Node] = []
 _pending_uses = {}   # id(leaf tensor) -> [tensor, outstanding uses]
 
@@ -207,18 +208,18 @@ def matmul(a: Tensor, b: Tensor) -> Tensor:
     out = Tensor.matmul(a, b)
 
     def grad_fn(g):
-        # On CUDA bf16 the transposed products run directly on the tensor cores (operand
-        # layout flags), no transposed copy is made.
+        # On CUDA the transposed products run directly on the tensor cores (operand layout
+        # flags), no transposed copy is made.
+        gt, at, bt = g._t, a._t, b._t
+        direct = gt.is_cuda and gt.dtype == at.dtype == bt.dtype and gt.dtype in _GEMM_DTYPES
+        if direct:
+            gt, at, bt = B._k(gt), B._k(at), B._k(bt)
         if a.requires_grad:
-            if g.device == "cuda" and g._t.dtype == torch.bfloat16:
-                acc_grad(a, B.gemm(g._t, b._t, b_t=True))
-            else:
-                acc_grad(a, Tensor.matmul(g, Tensor.transpose(b)))
+            acc_grad(a, B.gemm(gt, bt, b_t=True, out_dtype=gt.dtype) if direct
+                     else Tensor.matmul(g, Tensor.transpose(b)))
         if b.requires_grad:
-            if g.device == "cuda" and g._t.dtype == torch.bfloat16:
-                acc_grad(b, B.gemm(a._t, g._t, a_t=True))
-            else:
-                acc_grad(b, Tensor.matmul(Tensor.transpose(a), g))
+            acc_grad(b, B.gemm(at, gt, a_t=True, out_dtype=gt.dtype) if direct
+                     else Tensor.matmul(Tensor.transpose(a), g))
 
     record("matmul", [a, b], out, grad_fn)
     return out

@@ -1,0 +1,68 @@
+"""Products whose operands TMA cannot address (fp32, odd row lengths, narrow outputs): the direct
+kernel, the packed route and the SIMT kernel against a float64 reference.
+
+Bounds.  fp32: each operand loses at most 2^-18 of itself beyond its bf16 hi + lo parts and the
+lo * lo product (2^-18) is left out, so an element is off by at most 2^-16 sum|a||b|, plus fp32
+accumulation of 3 K terms, 3 K 2^-24 sum|a||b| worst case.  bf16 operands are exact: the rounding
+of the result (2^-8 of it) and the accumulation (K 2^-23 sum|a||b|) remain."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(1, 1, 1), (5, 3, 7), (16, 16, 512), (128, 64, 64), (129, 65, 65), (127, 63, 63), (256, 10, 784),
+         (61, 300, 2001), (257, 129, 1000), (1021, 1333, 777), (1, 1000, 300), (2049, 2047, 515)]
+
+
+def _check(out, a, b, dtype, extra=None):
+    ad, bd = a.double(), b.double()
+    ref = ad @ bd
+    mag = ad.abs() @ bd.abs()
+    K = a.shape[1]
+    if extra is not None:
+        ref, mag = ref + extra, mag + extra.abs()
+    bound = mag * (2.0 ** -16 + 3 * K * 2.0 ** -24) if dtype == torch.float32 else ref.abs() * 2.0 ** -8 + mag * K * 2.0 ** -23
+    assert bool(((out.double() - ref).abs() <= bound + 1e-30).all()), float(((out.double() - ref).abs() / (bound + 1e-30)).max())
+
+
+@pytest.mark.parametrize("M,N,K", SIZES)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("a_t,b_t", [(False, False), (False, True), (True, False), (True, True)])
+def test_any_operands(M, N, K, dtype, a_t, b_t):
+    from luatorch_b200 import _C, _backend as B
+    g = torch.Generator(device="cuda").manual_seed(M * 31 + N * 7 + K)
+    # odd offsets and row lengths: views into a larger buffer
+    def mat(rows, cols):
+        t = torch.randn(rows * (cols + 1) + 1, generator=g, device="cuda").to(dtype)
+        return t[1:].view(rows, cols + 1)[:, :cols]
+    a = mat(K, M) if a_t else mat(M, K)
+    b = mat(N, K) if b_t else mat(K, N)
+    out = B.gemm(a, b, a_t=a_t, b_t=b_t, out_dtype=dtype)
+    _check(out, a.t() if a_t else a, b.t() if b_t else b, dtype)
+    assert _C.gemm_device_error() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(33, 10, 300), (1021, 1333, 777)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_epilogue_and_repeatability(M, N, K, dtype):
+    """Bias, scale and accumulation, and the same bits twice."""
+    from luatorch_b200 import _backend as B
+    g = torch.Generator(device="cuda").manual_seed(5)
+    a, b = (torch.randn(s, generator=g, device="cuda").to(dtype) for s in ((M, K), (K, N)))
+    bias = torch.randn(N, generator=g, device="cuda")
+    outs = []
+    for _ in range(2):
+        out = torch.ones(M, N, device="cuda")
+        B.gemm(a, b, out=out, alpha=0.5, bias=bias, accumulate=True)
+        outs.append(out)
+    _check(outs[0], 0.5 * a, b, torch.float32, extra=(bias + 1.0).double().expand(M, N))
+    assert torch.equal(*outs)
+
+
+def test_batched_fp32():
+    from luatorch_b200 import _backend as B
+    g = torch.Generator(device="cuda").manual_seed(6)
+    a, b = torch.randn(5, 37, 70, generator=g, device="cuda"), torch.randn(5, 70, 131, generator=g, device="cuda")
+    out = B.bmm(a, b)
+    for i in range(5):
+        _check(out[i], a[i], b[i], torch.float32)
