@@ -6,12 +6,15 @@
 #include <c10/cuda/CUDAStream.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include <algorithm>
+#include <cmath>
 #include <map>
 #include <mutex>
 
 #include "../kernels/gemm.h"
 #include "../kernels/ops.h"
 #include "../kernels/attention.h"
+#include "../kernels/gpt_infer.h"
 #include "../comm/comm_kernels.h"
 
 namespace {
@@ -721,6 +724,82 @@ std::vector<Tensor> flash_backward(const Tensor& q, const Tensor& k, const Tenso
 }
 int64_t attention_device_error() { return lt::attention_last_device_error(); }
 
+// ------------------------------------------------------------------------------ GPT inference
+// `w`: tok, pos, lnf_g, lnf_b, head [embed, ld], then per layer ln1_g, ln1_b, wqkv, wo, bo, ln2_g,
+// ln2_b, w1, b1, w2, b2; bf16, matrices contiguous.
+lt::GptWeights gpt_weights(const std::vector<Tensor>& w, int64_t heads, int64_t vocab, double eps) {
+  TORCH_CHECK(w.size() >= 16 && (w.size() - 5) % 11 == 0, "gpt weights: 5 + 11 per layer expected");
+  lt::GptWeights g;
+  g.layers = (int)((w.size() - 5) / 11);
+  TORCH_CHECK(g.layers <= lt::GPT_MAX_LAYERS, "gpt weights: too many layers");
+  for (const Tensor& t : w)
+    TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.is_contiguous(), "gpt weights must be contiguous bf16 on the GPU");
+  g.tok = w[0].data_ptr(); g.pos = w[1].data_ptr(); g.lnf_g = w[2].data_ptr(); g.lnf_b = w[3].data_ptr();
+  g.head = w[4].data_ptr();
+  g.embed = (int)w[0].size(1);
+  g.heads = (int)heads; g.head_dim = g.embed / g.heads;
+  g.head_ld = w[4].size(1);
+  g.vocab = (int)vocab;
+  g.ffn = (int)w[5 + 7].size(1);
+  g.eps = (float)eps;
+  g.scale = 1.0f / std::sqrt((float)g.head_dim);
+  TORCH_CHECK(g.embed % 8 == 0 && g.ffn % 8 == 0 && g.head_ld % 8 == 0 && g.vocab <= g.head_ld &&
+              w[0].size(0) >= vocab && w[1].size(1) == g.embed, "gpt weights: unexpected shapes");
+  for (int l = 0; l < g.layers; ++l) {
+    const Tensor* t = &w[5 + 11 * l];
+    const int64_t E = g.embed, F = g.ffn;
+    const int64_t want[11] = {E, E, 3 * E * E, E * E, E, E, E, E * F, F, F * E, E};
+    for (int i = 0; i < 11; ++i) TORCH_CHECK(t[i].numel() == want[i], "gpt weights: unexpected shapes");
+    g.layer[l] = {t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), t[3].data_ptr(), t[4].data_ptr(), t[5].data_ptr(),
+                  t[6].data_ptr(), t[7].data_ptr(), t[8].data_ptr(), t[9].data_ptr(), t[10].data_ptr()};
+  }
+  return g;
+}
+Tensor bytes_like(const Tensor& like, size_t n) {
+  return at::empty({(int64_t)n}, like.options().dtype(at::kByte));
+}
+// logits [batch * seq, ld] of ids [batch * seq], and the status words of the embedding gather
+std::vector<Tensor> gpt_forward(const std::vector<Tensor>& w, int64_t heads, int64_t vocab, double eps,
+                                const Tensor& ids, int64_t batch, int64_t seq) {
+  need_cuda_contig(ids, "ids");
+  c10::cuda::CUDAGuard guard(ids.device());
+  const lt::GptWeights g = gpt_weights(w, heads, vocab, eps);
+  TORCH_CHECK(ids.numel() == batch * seq && seq <= w[1].size(0), "gpt_forward: sequence too long");
+  const int64_t T = batch * seq;
+  Tensor ws = bytes_like(ids, lt::gpt_forward_workspace(g, T));
+  Tensor logits = at::empty({T, g.head_ld}, w[0].options());
+  Tensor err = at::zeros({4}, ids.options().dtype(at::kInt));
+  void* x = nullptr;
+  check(lt::gpt_forward(g, ids.data_ptr(), label_kind(ids), batch, seq, ws.data_ptr(), nullptr, 0,
+                        err.data_ptr<int>(), &x, cur_stream()), "gpt_forward");
+  check(lt::gpt_logits(g, x, T, ws.data_ptr(), logits.data_ptr(), cur_stream()), "gpt_logits");
+  return {logits, err};
+}
+// rnd.numel() tokens sampled after `ids` (int32 on the device, followed by one status word)
+Tensor gpt_generate(const std::vector<Tensor>& w, int64_t heads, int64_t vocab, double eps, const Tensor& ids,
+                    const Tensor& rnd, double temperature, int64_t top_k) {
+  need_cuda_contig(ids, "ids"); need_cuda_contig(rnd, "rnd");
+  c10::cuda::CUDAGuard guard(ids.device());
+  const lt::GptWeights g = gpt_weights(w, heads, vocab, eps);
+  const int64_t S = ids.numel(), n = rnd.numel(), rows = S + n - 1;
+  TORCH_CHECK(S > 0 && n > 0 && rows <= w[1].size(0), "gpt_generate: sequence too long");
+  Tensor ws = bytes_like(ids, lt::gpt_forward_workspace(g, S));
+  Tensor cache = at::empty({g.layers, rows, 3 * g.embed}, w[0].options());
+  Tensor scratch = bytes_like(ids, lt::gpt_decode_scratch(g));
+  Tensor out = at::zeros({n + 1 + 4}, ids.options().dtype(at::kInt));   // ids | status | gather's words
+  int* o = out.data_ptr<int>();
+  void* x = nullptr;
+  check(lt::gpt_forward(g, ids.data_ptr(), label_kind(ids), 1, S, ws.data_ptr(), cache.data_ptr(), rows,
+                        o + n + 1, &x, cur_stream()), "gpt_forward");
+  const char* last = (const char*)x + (S - 1) * g.embed * 2;
+  // a few dozen tokens per launch: no kernel holds the GPU for long
+  for (int64_t i = 0; i < n; i += 32)
+    check(lt::gpt_decode(g, last, cache.data_ptr(), rows, (int)S, (int)i, (int)std::min(n, i + 32),
+                         (float)temperature, (int)top_k, rnd.data_ptr<float>(), o, scratch.data_ptr(), o + n,
+                         cur_stream()), "gpt_decode");
+  return out.slice(0, 0, n + 1);
+}
+
 // ------------------------------------------------------------------------------ comm kernels
 // Pointer tables are int64 CUDA tensors holding peer-mapped device addresses.
 void allreduce_adamw(const Tensor& grad_ptrs, const Tensor& signal_ptrs, int64_t rank,
@@ -839,6 +918,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("set_step_scalars", &set_step_scalars);
   m.def("flash_forward", &flash_forward);
   m.def("flash_backward", &flash_backward);
+  m.def("gpt_forward", &gpt_forward);
+  m.def("gpt_generate", &gpt_generate);
   m.def("attention_device_error", &attention_device_error);
   m.def("allreduce_adamw", &allreduce_adamw);
   m.def("peer_broadcast", &peer_broadcast);

@@ -33,6 +33,7 @@ KERNEL_SOURCES = [
     "kernels/gemm_tcgen05.cu", "kernels/gemm_direct.cu", "kernels/elementwise.cu", "kernels/reduce.cu",
     "kernels/softmax_ce.cu", "kernels/layernorm.cu", "kernels/embedding.cu", "kernels/conv.cu",
     "kernels/optim.cu", "kernels/attention_fwd.cu", "kernels/attention_bwd.cu",
+    "kernels/gpt_infer.cu",
     "comm/comm_kernels.cu",
 ]
 ABI_SOURCES = [

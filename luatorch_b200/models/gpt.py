@@ -3,15 +3,18 @@
 `GPT(vocab_size, embed_dim, num_heads, num_layers, max_seq_len, dropout=0.1)`: token
 embedding + positional encoding + embedding dropout + N pre-LN transformer blocks + final
 LayerNorm + UNTIED head Linear(embed, vocab, bias=False).  `forward(input[B, S])` returns
-logits [B*S, vocab]; `generate(prompt, max_tokens, temperature, top_k)` samples with a full
-re-forward per token, context cropped to `max_seq_len`; `parameters()` order is token_emb,
+logits [B*S, vocab]; `generate(prompt, max_tokens, temperature, top_k)` samples token by token,
+context cropped to `max_seq_len`; `parameters()` order is token_emb,
 positional (if learned), blocks, final_ln, head; `no_decay_params()` is every LayerNorm
 parameter plus the ffn1 / ffn2 / out_proj biases.
 
 Extension: `pos="learned"` selects a LearnedPE table (the reference always uses the fixed
 sinusoidal table).  On CUDA the token gather and the positional add are one kernel, and the
 head weight is stored with its row padded to a multiple of 8 columns so TMA can address the
-50257-wide vocabulary (checkpoints still hold the unpadded [embed, vocab] matrix).
+50257-wide vocabulary (checkpoints still hold the unpadded [embed, vocab] matrix).  Without
+gradients and in bf16 a forward is one native call, and `generate` is a prefill plus one
+persistent kernel over cached keys and values (csrc/kernels/gpt_infer.cu); once the context
+has to be cropped, every position changes and each token takes a full forward.
 """
 from __future__ import annotations
 
@@ -28,6 +31,7 @@ from ..nn.embedding import Embedding, embedding_backward_into
 from ..nn.layernorm import LayerNorm
 from ..nn.linear import Linear
 from ..nn.module import Module
+from ..nn.multihead import FlashMultiHeadAttention
 from ..nn.positional import LearnedPE, SinusoidalPE, positional_backward_into
 from ..nn.transformer import TransformerBlock
 from ..tensor import Tensor
@@ -84,9 +88,57 @@ class GPT(Module):
         x = self.token_emb(Tensor(_data=ids))
         return self.pos_enc(x, seq_len)
 
+    # ------------------------------------------------------------------ inference
+    def _inference_weights(self):
+        """The bf16 tensors the native inference path reads, or None where it does not apply
+        (CPU, fp32 compute, active dropout, other head sizes or block types)."""
+        emb = self.token_emb.weight
+        if not emb._t.is_cuda:
+            return None
+
+        def view(p):
+            t = p._compute if p._compute is not None else p._t
+            return t if t.dtype == torch.bfloat16 and t.is_contiguous() else None
+
+        if view(emb) is None or self.embed_dim // self.num_heads not in (64, 128):
+            return None
+        if isinstance(self.pos_enc, LearnedPE):
+            pos = view(self.pos_enc.weight)
+        else:
+            pos = self.pos_enc._table(view(emb))
+        head = self.head.weight_storage if self.head.weight_storage is not None else self.head.weight
+        ln = self.final_ln
+        out = [view(emb), pos, view(ln.gamma), view(ln.beta), view(head)]
+        if self.emb_drop.training and self.emb_drop.p > 0.0 or self.head.use_bias:
+            return None
+        for b in self.blocks:
+            a = b.attn
+            if (type(b) is not TransformerBlock or type(a) is not FlashMultiHeadAttention or not a.causal
+                    or a.num_heads != self.num_heads or b.ln1.eps != ln.eps or b.ln2.eps != ln.eps
+                    or b.training and (b.drop1.p > 0.0 or b.drop2.p > 0.0)
+                    or not (a.out_proj.use_bias and b.ffn1.use_bias and b.ffn2.use_bias)):
+                return None
+            out += [view(b.ln1.gamma), view(b.ln1.beta), view(a.qkv_weight), view(a.out_proj.weight),
+                    view(a.out_proj.bias), view(b.ln2.gamma), view(b.ln2.beta), view(b.ffn1.weight),
+                    view(b.ffn1.bias), view(b.ffn2.weight), view(b.ffn2.bias)]
+        if len(self.blocks) > 96 or any(t is None for t in out) or out[4].shape[1] % 8:
+            return None
+        return out
+
     def forward(self, input: Tensor) -> Tensor:
         shape = input.shape
         seq_len = shape[1] if len(shape) >= 2 else shape[0]
+        if not autograd.enabled and seq_len <= self.max_seq_len:
+            w = self._inference_weights()
+            if w is not None:
+                ids = input._t.reshape(-1)
+                ids = B._labels(ids if ids.is_cuda else ids.cuda())
+                logits, err = B.ext().gpt_forward(w, self.num_heads, self.vocab_size, self.final_ln.eps,
+                                                  ids, ids.numel() // seq_len, seq_len)
+                _debug.check_index_word(err, "GPT token embedding: token id")
+                if _debug._on:
+                    _debug.check_kernels(B.ext())
+                return Tensor(_data=logits[:, :self.vocab_size])
         x = self._embed(input._t.reshape(-1), seq_len)
         x = self.emb_drop(x)
         for block in self.blocks:
@@ -106,8 +158,21 @@ class GPT(Module):
         tokens = [int(v) for v in src.reshape(-1).tolist()]
         dev = self.token_emb.weight._t.device
         gen = B.cpu_generator()
+        todo = max_tokens or 100
         with autograd.no_grad():
-            for _ in range(max_tokens or 100):
+            w = self._inference_weights()
+            # cached keys and values serve until the context has to be cropped
+            n = min(todo, self.max_seq_len - len(tokens) + 1)
+            if w is not None and n > 0 and tokens:
+                rnd = torch.rand(n, generator=gen).to(dev)
+                ids = torch.tensor(tokens, dtype=torch.int32).to(dev)
+                got = B.ext().gpt_generate(w, self.num_heads, self.vocab_size, self.final_ln.eps, ids, rnd,
+                                           float(temperature), int(top_k)).tolist()
+                if got.pop() != 0:
+                    raise RuntimeError("GPT.generate: a grid-wide wait of the decode kernel ran out of time")
+                tokens += got
+                todo -= n
+            for _ in range(todo):
                 ctx = tokens[-self.max_seq_len:]
                 inp = Tensor(_data=torch.tensor(ctx, dtype=torch.float32, device=dev).reshape(1, -1))
                 autograd.zero_graph()

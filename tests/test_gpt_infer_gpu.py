@@ -1,0 +1,93 @@
+"""Native GPT inference (csrc/kernels/gpt_infer.cu) against the layer-by-layer path.
+
+The scoring forward issues the same kernels as the layers, so its logits are the same bits.  The
+decode kernel takes its sums in another order and keeps attention weights in fp32: a token it
+draws must lie within reach of the uniform number under the layer path's distribution for the
+same prefix, i.e. cdf(token - 1) - d <= r <= cdf(token) + d.  The logits here are below 16 in size
+and bf16, each off by at most an ulp or two (2 * 2^-5), so a cdf value p (1 - p) moves by at most
+0.25 * 2 * 2^-4 < d = 0.04."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _model(vocab, embed, heads, layers, max_seq, pos):
+    import luatorch_b200 as lf
+    lf.manual_seed(11)
+    m = lf.models.GPT(vocab, embed, heads, layers, max_seq, 0.0, pos=pos)
+    g = torch.Generator().manual_seed(3)
+    for b in m.blocks:
+        for lin in (b.attn.out_proj, b.ffn1, b.ffn2):
+            lin.bias._t.copy_(torch.randn(lin.bias._t.shape, generator=g) * 0.1)
+        for ln in (b.ln1, b.ln2):
+            ln.gamma._t.copy_(1 + 0.1 * torch.randn(ln.gamma._t.shape, generator=g))
+            ln.beta._t.copy_(0.1 * torch.randn(ln.beta._t.shape, generator=g))
+        for lin in (b.attn.out_proj, b.ffn2):
+            lin.weight._t.mul_((2 * layers) ** -0.5)
+    m.head.weight._t.mul_(0.5)
+    lf.cuda.amp.autocast_bf16(m)
+    return m.eval()
+
+
+def _layerwise(m, ids):
+    import luatorch_b200 as lf
+    native, m._inference_weights = m._inference_weights, lambda: None
+    try:
+        with lf.autograd.no_grad():
+            return m.forward(lf.Tensor.wrap(ids))._t
+    finally:
+        m._inference_weights = native
+
+
+@pytest.mark.parametrize("batch,seq", [(1, 1), (3, 77), (2, 128)])
+@pytest.mark.parametrize("embed,heads", [(128, 2), (256, 2)])
+def test_scoring_forward_is_the_layers(batch, seq, embed, heads):
+    import luatorch_b200 as lf
+    m = _model(331, embed, heads, 2, 128, "learned")
+    ids = torch.randint(0, 331, (batch, seq), device="cuda", dtype=torch.int32)
+    assert m._inference_weights() is not None
+    with lf.autograd.no_grad():
+        got = m.forward(lf.Tensor.wrap(ids))._t
+    assert got.shape == (batch * seq, 331)
+    assert torch.equal(got, _layerwise(m, ids))
+
+
+@pytest.mark.parametrize("vocab,embed,heads,layers,pos,prompt,n,temperature,top_k", [
+    (50257, 768, 12, 2, "learned", 100, 12, 0.8, 40),
+    (1000, 256, 4, 2, "sinusoidal", 17, 12, 1.0, 0),       # whole vocabulary
+    (777, 192, 3, 3, "learned", 1, 16, 1.3, 300),          # more than one CTA maximum per rank
+    (50257, 128, 2, 1, "learned", 250, 12, 1.0, 5000),     # across the fused-attention limit (256 keys)
+    (97, 64, 1, 1, "learned", 3, 9, 0.7, 5),               # fewer units than CTAs
+    (500, 256, 2, 2, "learned", 120, 14, 1.0, 20),         # head dim 128, across its limit (128 keys)
+    (333, 1280, 20, 1, "learned", 40, 6, 1.0, 50),         # more heads than K slices, wide residual
+])
+def test_decode_draws_from_the_layers_distribution(vocab, embed, heads, layers, pos, prompt, n, temperature, top_k):
+    import luatorch_b200 as lf
+    m = _model(vocab, embed, heads, layers, 300, pos)
+    ids = [(37 * i + 11) % vocab for i in range(prompt)]
+    lf.manual_seed(5)
+    toks = [int(t) for t in m.generate(ids, n, temperature, top_k).tolist()]
+    lf.manual_seed(5)
+    assert [int(t) for t in m.generate(ids, n, temperature, top_k).tolist()] == toks
+    assert toks[:prompt] == ids and len(toks) == prompt + n
+    lf.manual_seed(5)
+    rnd = torch.rand(n, generator=lf._backend.cpu_generator()).tolist()
+    full = torch.tensor([toks], dtype=torch.int32, device="cuda")
+    logits = _layerwise(m, full)[prompt - 1:-1].double() / temperature
+    for i in range(n):
+        v = logits[i]
+        if 0 < top_k < vocab:
+            v = torch.where(v < torch.topk(v, top_k).values[-1], torch.full_like(v, -float("inf")), v)
+        cdf = torch.cumsum(torch.softmax(v, 0), 0)
+        t = toks[prompt + i]
+        lo = float(cdf[t - 1]) if t else 0.0
+        assert lo - 0.04 <= rnd[i] <= float(cdf[t]) + 0.04, (i, t, lo, rnd[i], float(cdf[t]))
+
+
+def test_context_longer_than_the_model():
+    """Past max_seq_len the context is cropped and every token takes a forward of its own."""
+    import luatorch_b200 as lf
+    m = _model(97, 64, 1, 1, 24, "learned")
+    out = m.generate(list(range(20)), 12, 1.0, 3)
+    assert out.shape == [32] and all(0 <= int(t) < 97 for t in out.tolist())
