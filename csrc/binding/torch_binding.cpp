@@ -693,7 +693,8 @@ std::vector<Tensor> flash_backward(const Tensor& q, const Tensor& k, const Tenso
     dk = at::empty({B, S, H, D}, q.options());
     dv = at::empty({B, S, H, D}, q.options());
   }
-  Tensor delta = at::empty({B, H, S}, q.options().dtype(at::kFloat));
+  Tensor stats = at::empty({(int64_t)lt::flash_attention_backward_stats((int)B, (int)H, (int)S)},
+                           q.options().dtype(at::kFloat));
   lt::AttnArgs a;
   a.B = (int)B; a.H = (int)H; a.S = (int)S; a.D = (int)D;
   a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.o = (void*)o.data_ptr();
@@ -709,16 +710,7 @@ std::vector<Tensor> flash_backward(const Tensor& q, const Tensor& k, const Tenso
   b.dq_sb = dq.stride(0); b.dq_ss = dq.stride(1); b.dq_sh = dq.stride(2);
   b.dk_sb = dk.stride(0); b.dk_ss = dk.stride(1); b.dk_sh = dk.stride(2);
   b.dv_sb = dv.stride(0); b.dv_ss = dv.stride(1); b.dv_sh = dv.stride(2);
-  b.delta = delta.data_ptr<float>();
-  // scratch for the dS tiles (dQ = dS K as a GEMM).  Measured: worth it at head dim 128 (0.456
-  // vs 0.526 ms at B 4, S 2048, H 16), a wash at head dim 64 where writing and re-reading dS costs
-  // what the third kernel's recomputation costs.  LT_FLASH_DQ_GEMM=0 / 1 forces it off / on.
-  Tensor ds;
-  static const int dq_gemm = [] { const char* e = getenv("LT_FLASH_DQ_GEMM"); return e ? (e[0] == '0' ? 0 : 2) : 1; }();
-  if ((dq_gemm == 2 || (dq_gemm == 1 && D == 128)) && S % 128 == 0) {
-    ds = at::empty({B, H, S, S}, q.options());
-    b.ds_scratch = ds.data_ptr();
-  }
+  b.stats = stats.data_ptr<float>();
   check(lt::flash_attention_backward(a, b, cur_stream()), "flash_attention_backward");
   return {dq, dk, dv};
 }

@@ -12,7 +12,7 @@ namespace lt {
 
 // All tensors are bf16 with unit stride along head_dim and arbitrary element strides for
 // batch (sb), sequence (ss) and head (sh), so the [B*S, 3*E] output of a fused QKV
-// projection is consumed in place.  lse / delta are fp32 [B, H, S].
+// projection is consumed in place.  lse is fp32 [B, H, S].
 struct AttnArgs {
   int B = 0, H = 0, S = 0, D = 0;   // D in {64, 128}
   const void* q = nullptr; const void* k = nullptr; const void* v = nullptr;
@@ -33,14 +33,11 @@ struct AttnBwdArgs {
   int64_t dq_sb = 0, dq_ss = 0, dq_sh = 0;
   int64_t dk_sb = 0, dk_ss = 0, dk_sh = 0;
   int64_t dv_sb = 0, dv_ss = 0, dv_sh = 0;
-  float* delta = nullptr;           // scratch [B, H, S]: rowsum(dO * O)
-  // Optional bf16 scratch [B, H, S, S].  When given (and S is a multiple of 128) the dK/dV
-  // kernel also writes its dS tiles there and dQ = dS K runs as a batched tensor-core GEMM
-  // over them instead of a third kernel that would rebuild S, dP and dS a second time.
-  void* ds_scratch = nullptr;
+  float* stats = nullptr;           // scratch, flash_attention_backward_stats() floats, 16-byte aligned
 };
 
 cudaError_t flash_attention_forward(const AttnArgs& a, cudaStream_t stream);
+size_t flash_attention_backward_stats(int B, int H, int S);   // floats of AttnBwdArgs::stats
 cudaError_t flash_attention_backward(const AttnArgs& a, const AttnBwdArgs& b, cudaStream_t stream);
 
 int attention_last_device_error();
