@@ -912,6 +912,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("flash_backward", &flash_backward);
   m.def("gpt_forward", &gpt_forward);
   m.def("gpt_generate", &gpt_generate);
+  m.def("gpt_decode_fits", &lt::gpt_decode_fits);
   m.def("attention_device_error", &attention_device_error);
   m.def("allreduce_adamw", &allreduce_adamw);
   m.def("peer_broadcast", &peer_broadcast);

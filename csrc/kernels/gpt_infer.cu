@@ -251,6 +251,7 @@ struct VecSlice {
   }
 };
 
+constexpr int DECODE_SMEM_MAX = 200 * 1024;   // beside about 17 KB of static shared memory
 // Shared memory of the decode kernel (floats): slots | x | n | slice | red.
 __host__ __device__ inline int decode_smem_floats(int E, int F) {
   const int wide = E > F ? E : F;
@@ -785,6 +786,13 @@ cudaError_t gpt_logits(const GptWeights& w, const void* x, int64_t n, void* work
   return e;
 }
 
+bool gpt_decode_fits(int64_t embed, int64_t ffn, int64_t head_dim, int64_t vocab) {
+  const int64_t wide = embed > ffn ? embed : ffn;
+  if ((head_dim != 64 && head_dim != 128) || wide > (1 << 20) || vocab * embed >= (1ll << 31)) return false;
+  // a head's sums and its context vector share the activations' buffer
+  return decode_smem_floats((int)embed, (int)ffn) * 4 <= DECODE_SMEM_MAX && 2 * head_dim + 2 <= wide;
+}
+
 size_t gpt_decode_scratch(const GptWeights& w) {
   const int G = sm_count();
   return (size_t)(256 + up((int64_t)MAX_KS * w.embed * 4) +
@@ -795,11 +803,10 @@ size_t gpt_decode_scratch(const GptWeights& w) {
 cudaError_t gpt_decode(const GptWeights& w, const void* x, void* cache, int64_t cache_rows, int prompt,
                        int first, int last, float temperature, int top_k, const float* rnd, int* ids_out,
                        void* scratch, int* status, cudaStream_t s) {
-  if (w.head_dim != 64 && w.head_dim != 128) return cudaErrorInvalidValue;
+  if (!gpt_decode_fits(w.embed, w.ffn, w.head_dim, w.vocab)) return cudaErrorInvalidValue;
   const int smem = decode_smem_floats(w.embed, w.ffn) * 4;
-  static const cudaError_t attr = cudaFuncSetAttribute(gpt_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  static const cudaError_t attr = cudaFuncSetAttribute(gpt_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DECODE_SMEM_MAX);
   if (attr != cudaSuccess) return attr;
-  if (smem > 200 * 1024) return cudaErrorInvalidValue;
   int G = sm_count();
   DecodeParams p;
   p.w = w;

@@ -40,6 +40,8 @@ cudaError_t gpt_logits(const GptWeights& w, const void* x, int64_t n, void* work
 // is the residual stream of the prompt's last position (used for i == 0), `cache` the prompt's
 // q | k | v rows with room for the new ones.  `scratch`: gpt_decode_scratch() bytes.  status[0]
 // is set when a grid-wide wait ran out of time.
+// A model fits when its vectors do (shared memory) and table offsets stay below 2^31.
+bool gpt_decode_fits(int64_t embed, int64_t ffn, int64_t head_dim, int64_t vocab);
 size_t gpt_decode_scratch(const GptWeights& w);
 cudaError_t gpt_decode(const GptWeights& w, const void* x, void* cache, int64_t cache_rows, int prompt,
                        int first, int last, float temperature, int top_k, const float* rnd, int* ids_out,

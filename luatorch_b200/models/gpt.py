@@ -91,7 +91,7 @@ class GPT(Module):
     # ------------------------------------------------------------------ inference
     def _inference_weights(self):
         """The bf16 tensors the native inference path reads, or None where it does not apply
-        (CPU, fp32 compute, active dropout, other head sizes or block types)."""
+        (CPU, fp32 compute, active dropout, other head sizes, layers of other types)."""
         emb = self.token_emb.weight
         if not emb._t.is_cuda:
             return None
@@ -111,10 +111,17 @@ class GPT(Module):
         out = [view(emb), pos, view(ln.gamma), view(ln.beta), view(head)]
         if self.emb_drop.training and self.emb_drop.p > 0.0 or self.head.use_bias:
             return None
+        if (type(self.token_emb) is not Embedding or type(self.pos_enc) not in (LearnedPE, SinusoidalPE)
+                or type(self.emb_drop) is not Dropout or type(ln) is not LayerNorm or type(self.head) is not Linear):
+            return None
+        scale = 1.0 / math.sqrt(self.embed_dim // self.num_heads)
         for b in self.blocks:
             a = b.attn
             if (type(b) is not TransformerBlock or type(a) is not FlashMultiHeadAttention or not a.causal
-                    or a.num_heads != self.num_heads or b.ln1.eps != ln.eps or b.ln2.eps != ln.eps
+                    or a.num_heads != self.num_heads or a.scale != scale
+                    or any(type(m) is not LayerNorm or m.eps != ln.eps for m in (b.ln1, b.ln2))
+                    or any(type(m) is not Linear for m in (a.out_proj, b.ffn1, b.ffn2))
+                    or any(type(m) is not Dropout for m in (b.drop1, b.drop2))
                     or b.training and (b.drop1.p > 0.0 or b.drop2.p > 0.0)
                     or not (a.out_proj.use_bias and b.ffn1.use_bias and b.ffn2.use_bias)):
                 return None
@@ -124,6 +131,15 @@ class GPT(Module):
         if len(self.blocks) > 96 or any(t is None for t in out) or out[4].shape[1] % 8:
             return None
         return out
+
+    def _decode_applies(self, w, temperature) -> bool:
+        """Whether the decode kernel stands for a loop over `forward`: nobody has replaced that
+        method, the model fits the kernel's shared memory, the temperature keeps the order of
+        the logits, and nobody asked for the checks that follow every launch."""
+        return (getattr(self.forward, "__func__", None) is GPT.forward and not _debug._on
+                and 0.0 < temperature < math.inf
+                and B.ext().gpt_decode_fits(self.embed_dim, w[5 + 7].shape[1],
+                                            self.embed_dim // self.num_heads, self.vocab_size))
 
     def forward(self, input: Tensor) -> Tensor:
         shape = input.shape
@@ -163,7 +179,7 @@ class GPT(Module):
             w = self._inference_weights()
             # cached keys and values serve until the context has to be cropped
             n = min(todo, self.max_seq_len - len(tokens) + 1)
-            if w is not None and n > 0 and tokens:
+            if w is not None and n > 0 and tokens and self._decode_applies(w, temperature):
                 rnd = torch.rand(n, generator=gen).to(dev)
                 ids = torch.tensor(tokens, dtype=torch.int32).to(dev)
                 got = B.ext().gpt_generate(w, self.num_heads, self.vocab_size, self.final_ln.eps, ids, rnd,

@@ -85,6 +85,43 @@ def test_decode_draws_from_the_layers_distribution(vocab, embed, heads, layers, 
         assert lo - 0.04 <= rnd[i] <= float(cdf[t]) + 0.04, (i, t, lo, rnd[i], float(cdf[t]))
 
 
+def test_decode_kernel_only_stands_for_the_stock_loop():
+    """Models and options that the decode kernel does not cover keep the loop over `forward`."""
+    import luatorch_b200 as lf
+    from luatorch_b200 import _C
+    calls = []
+
+    class Counting(lf.models.GPT):
+        def forward(self, x):
+            calls.append(x.shape)
+            return super().forward(x)
+
+    class Scaled(lf.nn.Linear):
+        def forward(self, *args, **kwargs):
+            calls.append(None)
+            return super().forward(*args, **kwargs)
+
+    def seen(m, temperature=1.0):
+        calls.clear()
+        out = m.generate([1, 2, 3], 3, temperature, 5)
+        assert out.shape == [6] and all(0 <= int(t) < 97 for t in out.tolist())
+        return len(calls)
+
+    m = Counting(97, 128, 2, 1, 24, 0.0)
+    lf.cuda.amp.autocast_bf16(m)
+    assert seen(m.eval()) == 3
+    m = _model(97, 128, 2, 1, 24, "learned")
+    assert seen(m) == 0 and m._inference_weights() is not None
+    w = m._inference_weights()
+    assert not m._decode_applies(w, -1.0) and not m._decode_applies(w, 0.0) and not m._decode_applies(w, float("nan"))
+    assert m._decode_applies(w, 0.5)
+    assert seen(m, -1.0) == 0                                 # the loop, over the stock forward
+    m.blocks[0].ffn1.__class__ = Scaled
+    assert m._inference_weights() is None and seen(m) == 3
+    # 24 bytes of shared memory per embedding column beside 100 KB of weight slots
+    assert _C.gpt_decode_fits(4096, 16384, 128, 50257) and not _C.gpt_decode_fits(4608, 18432, 128, 50257)
+
+
 def test_context_longer_than_the_model():
     """Past max_seq_len the context is cropped and every token takes a forward of its own."""
     import luatorch_b200 as lf
