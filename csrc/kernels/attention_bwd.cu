@@ -63,8 +63,8 @@ struct BwdParams {
 // can be fetched by bulk copies (16-byte aligned, never past the end).  A padded query gets
 // lse = +inf: its probabilities are exp2(-inf) = 0 and nothing else has to mask it.
 // D / 8 lanes share a query (16-byte loads, whole lines), 32 queries of one head per CTA.
-// Bound by memory; [8, 1024, 12, 64] takes 6.1 us (8.8 with a thread per query and strided loads),
-// [4, 2048, 16, 128] 12.0 us (21.7).
+// Bound by memory; [8, 1024, 12, 64] takes 7.1 us (8.8 with a thread per query and strided loads),
+// [4, 2048, 16, 128] 13.1 us (21.7).
 constexpr int STAT_ROWS = 32;
 template <int D>
 __global__ void __launch_bounds__(STAT_ROWS * 8)
@@ -76,7 +76,7 @@ attn_stats_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
   constexpr int PARTS = D / 64;              // 16-byte loads per lane: 8 lanes per query
   const int h = blockIdx.x, b = blockIdx.y;
   const int s = (int)blockIdx.z * STAT_ROWS + (threadIdx.x >> 3), v = threadIdx.x & 7;
-  float acc = 0.0f;
+  float t[PARTS][4] = {};
   if (s < S) {
     const __nv_bfloat16* op = o + b * o_sb + s * o_ss + h * o_sh + v * 8;
     const __nv_bfloat16* dp = d_o + b * do_sb + s * do_ss + h * do_sh + v * 8;
@@ -93,12 +93,20 @@ attn_stats_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float2 a = __bfloat1622float2(xh[j]), c = __bfloat1622float2(yh[j]);
-        acc += a.x * c.x + a.y * c.y;
+        t[i][j] = a.x * c.x + a.y * c.y;
       }
     }
   }
+  // added in the order of d, the sum handed from lane to lane
+  float acc = 0.0f;
 #pragma unroll
-  for (int m = 4; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+  for (int i = 0; i < PARTS; ++i)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const float sum = __shfl_sync(0xffffffffu, acc, (q + 7) & 7, 8);
+      if (v == q) acc = sum + t[i][0] + t[i][1] + t[i][2] + t[i][3];
+    }
+  acc = __shfl_sync(0xffffffffu, acc, 7, 8);
   if (v == 0) {
     const long long bh = (long long)b * H + h, at = bh * Sp + s;
     lse2[at] = s < S ? lse[bh * S + s] * LOG2E : INFINITY;
@@ -149,8 +157,11 @@ __device__ __forceinline__ void store_acc_row(uint32_t taddr, __nv_bfloat16* dst
 // memory, so two CTAs share an SM and one CTA's exponentials run under the other's MMAs.  At head
 // dim 128 only one CTA fits; there S and dP have two buffers (2 x 128 + 2 x 128 = all 512 columns)
 // and the MMAs of step i + 1 are issued before the exponentials of step i have come back.
-// Bound by the rate of tcgen05.mma at N = 64 (70 to 100 cycles each instead of 32).
-// All three launches, causal: [4, 1000, 12, 64] 83 -> 69 us, [4, 2048, 16, 128] 426 -> 376 us, against
+// Bound by the chain MMA -> barrier -> TMEM load -> exponentials -> TMEM store -> barrier -> MMA (about
+// 2500 cycles per step; issue slots, tensor pipe and MUFU are all below a third).  Tiles of 128
+// streamed rows with a barrier each for S, P, dP and dS, so that P dO and dS Q alternate with the
+// exponentials of one CTA, took the same time at head dim 128 and 5 % more at 64.
+// All three launches, causal: [4, 1000, 12, 64] 83 -> 61 us, [4, 2048, 16, 128] 426 -> 299 us, against
 // kernels that staged P and dS through shared memory (and dS through 0.5 GB of device memory).
 //
 // Lengths that are no multiple of a tile: TMA fills the missing rows with zeros, a missing query has
@@ -230,7 +241,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_fix0, const __grid_const
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
-  const int warp_idx = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp_idx = warp_index(), lane = threadIdx.x & 31;
   const int h = blockIdx.x, b = blockIdx.y;
   const int n_sub = (p.S + SUB - 1) / SUB;
   const int own = DKDV ? (int)blockIdx.z : (int)gridDim.z - 1 - (int)blockIdx.z;  // longest first
@@ -280,7 +291,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_fix0, const __grid_const
   auto str1 = [&](int st) { return smem + L::OFF_STR + st * 2 * L::STR + L::STR; };
 
   if (warp_idx == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t fb = smem_u32(fix_full);
       mbar_arrive_expect_tx(fb, 2 * L::FIX);
 #pragma unroll
@@ -310,7 +321,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_fix0, const __grid_const
       }
     }
   } else if (warp_idx == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_s = make_idesc_bf16(BT, SUB, 0, 0);   // [128 lanes] x [64 streamed rows]
       const uint32_t idesc_acc = make_idesc_bf16(BT, D, 0, 1);   // A from TMEM, B = streamed tile, rows as K
       bool ok = mbar_wait_bounded(smem_u32(fix_full), 0, abort_flag, &g_attn_error, 72);

@@ -193,7 +193,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 14);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
-  const int warp_idx = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp_idx = warp_index(), lane = threadIdx.x & 31;
   // longest (most key tiles) query tiles first
   const int q_tile = (int)gridDim.z - 1 - (int)blockIdx.z;
   const int h = blockIdx.x, b = blockIdx.y;
@@ -232,7 +232,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const uint32_t tmem_o = tmem_base + NSB * 128;    // D columns
 
   if (warp_idx == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t qb = smem_u32(q_full);
       mbar_arrive_expect_tx(qb, L::Q_BYTES);
 #pragma unroll
@@ -257,7 +257,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
     }
   } else if (warp_idx == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_s = make_idesc_bf16(BM, BN, 0, 0);
       const uint32_t idesc_o = make_idesc_bf16(BM, D, 0, 1);
       bool ok = mbar_wait_bounded(smem_u32(q_full), 0, abort_flag, &g_attn_error, 12);
@@ -588,7 +588,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 11);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
-  const int warp_idx = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp_idx = warp_index(), lane = threadIdx.x & 31;
   const int q_tile = (int)gridDim.z - 1 - (int)blockIdx.z;   // longest tiles first, over the WHOLE grid
   const int h = blockIdx.x, b = blockIdx.y;
   const int q0 = q_tile * BM;
@@ -625,7 +625,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const uint32_t tmem_o = tmem_base + 128;
 
   if (warp_idx == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t qb = smem_u32(q_full);
       mbar_arrive_expect_tx(qb, L::TILE);
 #pragma unroll
@@ -650,7 +650,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       }
     }
   } else if (warp_idx == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_s = make_idesc_bf16(BM, BN, 0, 0);
       const uint32_t idesc_o = make_idesc_bf16(BM, D, 0, 1);
       bool ok = mbar_wait_bounded(smem_u32(q_full), 0, abort_flag, &g_attn_error, 52);

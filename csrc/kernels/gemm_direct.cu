@@ -178,7 +178,7 @@ gemm_direct_kernel(const DirectParams d, const KernelParams p) {
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int S = d.splits;
   const int rank = S > 1 ? (int)cluster_cta_rank() : 0;
   const int tile = (int)blockIdx.x / S;
@@ -263,7 +263,7 @@ gemm_direct_kernel(const DirectParams d, const KernelParams p) {
       }
       tc_fence_before_sync();
     }
-  } else if (lane == 0) {
+  } else if (elect_one()) {
     const uint32_t idesc = make_idesc_bf16(BM, BN, A_MN, B_MN);
     constexpr uint32_t a_lbo = A_MN ? 64 * BK * 2 : 16, b_lbo = B_MN ? 64 * BK * 2 : 16;
     constexpr uint32_t a_step = A_MN ? (2048 >> 4) : (32 >> 4), b_step = B_MN ? (2048 >> 4) : (32 >> 4);

@@ -392,7 +392,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
   uint32_t* tmem_base_holder = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_holder + 1);
 
-  const int warp_idx = threadIdx.x >> 5;
+  const int warp_idx = warp_index();
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -443,7 +443,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   if (warp_idx == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -503,7 +503,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
   } else if (warp_idx == 1) {
     // ------------------------------- MMA issuer -------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_bf16(BM, BN, p.a_mn, p.b_mn);
       // K-major: 8-row groups 1024 B apart, k-step of 16 elements = 32 B inside the span.
       // MN-major: 64-element chunks 64*BK*2 B apart (LBO), 8-k groups 1024 B apart (SBO),
@@ -757,7 +757,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_holder + 1);
   int* gather_fail = reinterpret_cast<int*>(tmem_base_holder + 2);
 
-  const int warp_idx = threadIdx.x >> 5;
+  const int warp_idx = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t cta_rank = cluster_cta_rank();   // 0 = even CTA (issues the MMAs), 1 = odd
   const int cluster_id = blockIdx.x >> 1;
@@ -796,7 +796,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   if (warp_idx == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -879,7 +879,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
   } else if (warp_idx == 1) {
     // ----------------------- MMA issuer (even CTA only) -----------------------
-    if (lane == 0 && cta_rank == 0) {
+    if (cta_rank == 0 && elect_one()) {
       const uint32_t idesc = make_idesc_bf16(2 * BM, BN, p.a_mn, p.b_mn);
       const uint32_t a_lbo = p.a_mn ? 64 * BK * 2 : 16, b_lbo = p.b_mn ? 64 * BK * 2 : 16;
       const uint32_t a_step = p.a_mn ? (2048 >> 4) : (32 >> 4);
