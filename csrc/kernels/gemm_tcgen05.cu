@@ -1414,26 +1414,52 @@ cudaError_t launch_choice(const TileChoice& t, const GemmArgs& a, cudaStream_t s
   }
 }
 
-// C = sum_s ws[s] (+ bias) (+ C), four elements per thread; slices are added in index order.
+// C = sum_s ws[s] (+ bias) (+ C), four elements per thread.  SG warps share the slices of their
+// elements (warp g adds slices g, g + SG, ...) and the first adds the SG sums: a fixed order.
 // The workspace rows are `ws_ld` floats apart (N rounded up to 4); C is written with 16-byte
 // accesses when `vec` says its rows allow it, element by element otherwise (N = 27 ...).
+// Bound by latency: a convolution's weight gradient has up to 148 slices of a few thousand elements;
+// one thread walking all of them took 11.4 us a call (four in the convolution net), eight 3.7.
+template <int SG>
 __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(const float* __restrict__ ws, int splits, long long slice, int M, int N,
                      int ws_ld, void* C, long long ldc, int c_fp32, int accumulate,
                      const void* __restrict__ bias, int bias_fp32, int vec) {
+  constexpr int QB = 256 / SG;                // quads per block and turn
+  __shared__ float4 sh[SG > 1 ? SG : 1][SG > 1 ? QB : 1];
   pdl_enter();
   const int qpr = ws_ld / 4;
   const long long quads = (long long)M * qpr;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < quads;
-       q += (long long)gridDim.x * blockDim.x) {
+  const int g = threadIdx.x / QB, t = threadIdx.x % QB;
+  for (long long q0 = blockIdx.x * (long long)QB; q0 < quads; q0 += (long long)gridDim.x * QB) {
+    const long long q = q0 + t;
     const long long row = q / qpr;
     const int col = (int)(q - row * qpr) * 4;
-    const float* src = ws + row * ws_ld + col;
-    float4 acc = *reinterpret_cast<const float4*>(src);
-    for (int s = 1; s < splits; ++s) {
-      const float4 v = *reinterpret_cast<const float4*>(src + s * slice);
-      acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (q < quads) {
+      const float* src = ws + row * ws_ld + col;
+      for (int s0 = g; s0 < splits; s0 += 8 * SG) {   // eight loads in flight, added in order
+        float4 v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          v[k] = s0 + k * SG < splits ? *reinterpret_cast<const float4*>(src + (s0 + k * SG) * slice)
+                                      : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { acc.x += v[k].x; acc.y += v[k].y; acc.z += v[k].z; acc.w += v[k].w; }
+      }
     }
+    if constexpr (SG > 1) {
+      __syncthreads();                        // the turn before has been read
+      sh[g][t] = acc;
+      __syncthreads();
+      if (g > 0) continue;
+#pragma unroll
+      for (int k = 1; k < SG; ++k) {
+        const float4 v = sh[k][t];
+        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+      }
+    }
+    if (q >= quads) continue;
     float r[4] = {acc.x, acc.y, acc.z, acc.w};
     if (bias) {
 #pragma unroll
@@ -1591,9 +1617,12 @@ cudaError_t gemm_bf16(const GemmArgs& args, cudaStream_t stream) {
   cudaError_t e = launch_choice(tile, g, stream);
   if (e != cudaSuccess) return e;
   const long long quads = (long long)a.M * (ws_ld / 4);
-  int blocks = (int)((quads + 255) / 256);
+  // eight warps per element where there are slices for them and too few elements to fill the chip
+  const bool shared = splits > 8 && quads < 32ll * 8 * num_sms();
+  const int per_block = shared ? 32 : 256;
+  int blocks = (int)((quads + per_block - 1) / per_block);
   if (blocks > 8 * num_sms()) blocks = 8 * num_sms();
-  cudaError_t re = launch_pdl(splitk_reduce_kernel, dim3(blocks), dim3(256), 0, stream,
+  cudaError_t re = launch_pdl(shared ? splitk_reduce_kernel<8> : splitk_reduce_kernel<1>, dim3(blocks), dim3(256), 0, stream,
                               (const float*)a.workspace, splits, (long long)a.M * ws_ld, a.M, a.N,
                               ws_ld, a.C, (long long)a.ldc, a.c_fp32, a.accumulate, a.bias,
                               a.bias_fp32, reduce_vec_ok(a) ? 1 : 0);
