@@ -81,14 +81,18 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
   return v;
 }
 
-// All CTAs of the (cooperative) grid.  `goal` counts arrivals over the kernel's life.  Returns
-// false, for every thread of the CTA, when the wait ran out of time anywhere.
-__device__ bool grid_barrier(unsigned* bar, unsigned& goal, int* status, int* sh_ok) {
+// Barrier over all CTAs of the (cooperative) grid, in two halves: what a CTA does between them (asking
+// for the next weights: 600 to 2000 cycles of issue per phase) nobody waits for.  `goal` counts
+// arrivals over the kernel's life.
+__device__ void grid_arrive(unsigned* bar, unsigned& goal) {
   __syncthreads();
   goal += gridDim.x;
+  // release at gpu scope: covers what the whole CTA wrote before the __syncthreads
+  if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+}
+// Returns false, for every thread of the CTA, when the wait ran out of time anywhere.
+__device__ bool grid_wait(unsigned* bar, unsigned goal, int* status, int* sh_ok) {
   if (threadIdx.x == 0) {
-    // release at gpu scope: covers what the whole CTA wrote before the __syncthreads
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
     const long long t0 = clock64();
     int ok = 1;
     for (unsigned spin = 0; (int)(ld_acquire(bar) - goal) < 0; ++spin) {
@@ -114,6 +118,7 @@ __device__ __forceinline__ void prefetch_l2(const void* p, long long bytes) {
 // t / groups; each CTA takes tasks blockIdx.x, + gridDim.x, ...  A thread multiplies unit u (8
 // columns) of every RP-th row of the slice.  Lives in shared memory; the geometry of the CTA's
 // first task is the same in every layer.
+constexpr int FETCH = 24;    // weight slots per thread, see fetch()
 struct Product {
   int ldw, K, N, lg, tasks;
   Split sp;
@@ -132,20 +137,24 @@ struct Product {
     n = (slice + 1 == sp.ks ? K : (len * (slice + 1)) & ~7) - k0;
   }
   // this thread's first weight and its number of rows
-  __device__ __forceinline__ int rows(long long& off) const {
-    const int u = u0 + ((int)threadIdx.x & (sp.nu - 1)), r = threadIdx.x >> lg, RP = DT >> lg;
+  __device__ __forceinline__ int rows(long long& off) const { return rows_at(off, u0); }
+  __device__ __forceinline__ int rows_at(long long& off, int first_unit) const {
+    const int u = first_unit + ((int)threadIdx.x & (sp.nu - 1)), r = threadIdx.x >> lg, RP = DT >> lg;
     off = (long long)(k0 + r) * ldw + u * 8;
     return u * 8 < N && r < n ? (n - r + RP - 1) >> (31 - __clz(RP)) : 0;
+  }
+  // several tasks per CTA, all over the whole of K, whose weights fit half of the slots
+  __device__ __forceinline__ bool streamed() const {
+    const int RP = DT >> lg;
+    return sp.ks == 1 && tasks > (int)gridDim.x && (K + RP - 1) / RP <= FETCH / 2;
   }
 };
 
 // The first weights of this CTA's first task, copied into shared memory (a 16-byte slot per thread
 // and row) before the barrier that the activations wait for: their latency hides behind it.
-constexpr int FETCH = 24;
-__device__ __noinline__ void fetch(const Product& p, const void* W, uint4* slots) {
-  if ((int)blockIdx.x >= p.tasks) return;
+__device__ __noinline__ void fetch(const Product& p, const void* W, uint4* slots, int first_unit) {
   long long off;
-  int cnt = p.rows(off);
+  int cnt = p.rows_at(off, first_unit);
   if (cnt > FETCH) cnt = FETCH;
   const bf16* q = reinterpret_cast<const bf16*>(W) + off;
   const long long step = (long long)(DT >> p.lg) * p.ldw;
@@ -153,6 +162,10 @@ __device__ __noinline__ void fetch(const Product& p, const void* W, uint4* slots
 #pragma unroll 4
   for (int i = 0; i < cnt; ++i, q += step, dst += DT * 16)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(q) : "memory");
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void fetch(const Product& p, const void* W, uint4* slots) {
+  if ((int)blockIdx.x < p.tasks) fetch(p, W, slots, p.u0);
 }
 
 __device__ __forceinline__ void add8(float2 (&acc)[4], const uint4& v, float x) {
@@ -164,16 +177,19 @@ __device__ __forceinline__ void add8(float2 (&acc)[4], const uint4& v, float x) 
 }
 
 // Sums of the current task: `xs` are the activations of its K slice; column c < 8 nu of the task ends
-// up in thread c.  Sums are taken in a fixed order.  `slots`: its first weights, or null.
-__device__ __noinline__ float dot_task(const Product& p, const void* W, const uint4* slots, const float* xs,
-                                       float* red) {
+// up in thread c.  Sums are taken in a fixed order.  `slots`: its first weights, or null; `behind`: one
+// more group of copies has been started after them.
+__device__ __noinline__ float dot_task(const Product& p, const void* W, const uint4* slots, bool behind,
+                                       const float* xs, float* red) {
   float2 acc[4] = {};
   long long off;
   const int cnt = p.rows(off), RP = DT >> p.lg;
   const float* x = xs + (threadIdx.x >> p.lg);
   int i = 0;
   if (slots) {
-    asm volatile("cp.async.wait_all;" ::: "memory");   // a thread reads the slots it filled itself
+    // a thread reads the slots it filled itself
+    if (behind) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else asm volatile("cp.async.wait_all;" ::: "memory");
     const uint4* q = slots + threadIdx.x;
     const int m = cnt < FETCH ? cnt : FETCH;
 #pragma unroll 4
@@ -214,17 +230,24 @@ __device__ __noinline__ float dot_task(const Product& p, const void* W, const ui
 // Runs this CTA's tasks: `load(k0, n)` gives the activations of a K slice, `emit(slice, column, sum)`
 // takes every finished sum.
 template <typename Load, typename Emit>
-__device__ __forceinline__ void product(Product& p, const void* W, const uint4* slots, float* red, Load load,
+__device__ __forceinline__ void product(Product& p, const void* W, uint4* slots, float* red, Load load,
                                         Emit emit) {
   const int c = threadIdx.x;
+  const bool streamed = p.streamed();
+  int half = 0;                                // streamed: the half of the slots this task's weights are in
   for (int t = blockIdx.x; t < p.tasks; t += gridDim.x) {
     const bool first = t == (int)blockIdx.x;
+    const bool behind = streamed && t + (int)gridDim.x < p.tasks;
+    // the next task's weights arrive under this one's sums
+    if (behind) fetch(p, W, slots + (half ^ 1) * (FETCH / 2) * DT, (t + (int)gridDim.x) * p.sp.nu);
     if (!first) {
       __syncthreads();
       if (c == 0) p.select(t);
       __syncthreads();
     }
-    const float s = dot_task(p, W, first ? slots : nullptr, load(p.k0, p.n), red);
+    const float s = dot_task(p, W, first || streamed ? slots + half * (FETCH / 2) * DT : nullptr, behind,
+                             load(p.k0, p.n), red);
+    half ^= streamed;
     if (c < p.sp.nu * 8 && p.u0 * 8 + c < p.N) emit(p.slice, p.u0 * 8 + c, s);
   }
   if ((int)(blockIdx.x + gridDim.x) < p.tasks) {   // back to the first task
@@ -237,6 +260,7 @@ __device__ __forceinline__ void product(Product& p, const void* W, const uint4* 
 // The elements of a vector parameter that this thread handles (e = thread, + DT, ...), loaded
 // ahead like the weights; longer vectors load the rest where they are used.
 constexpr int EPT = 3;
+constexpr int NORM_V = 8;            // 16-byte vectors per lane when a warp norms the whole stream
 struct VecSlice {
   const void* p;
   bf16 v[EPT];
@@ -374,6 +398,34 @@ __global__ void __launch_bounds__(DT, 1) gpt_decode_kernel(const __grid_constant
   const float inv_e = 1.0f / E;
   // element e = tid + i DT of the residual stream belongs to this thread
   auto norm = [&]() {
+    if (E <= 32 * 4 * NORM_V) {
+      // every warp sums the whole vector: two shuffle trees and no block-wide sums
+      __syncthreads();
+      const int lane = tid & 31;
+      float4 t[NORM_V];
+      float s = 0.0f, q = 0.0f;
+#pragma unroll
+      for (int i = 0; i < NORM_V; ++i) {
+        const int e = (lane + 32 * i) * 4;
+        t[i] = e < E ? *reinterpret_cast<const float4*>(x + e) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        s += (t[i].x + t[i].y) + (t[i].z + t[i].w);
+      }
+      const float mean = warp_sum(s) * inv_e;
+#pragma unroll
+      for (int i = 0; i < NORM_V; ++i) {
+        const float a = t[i].x - mean, b = t[i].y - mean, c = t[i].z - mean, d = t[i].w - mean;
+        if ((lane + 32 * i) * 4 < E) q += (a * a + b * b) + (c * c + d * d);
+      }
+      const float rstd = rsqrtf(warp_sum(q) * inv_e + w.eps);
+#pragma unroll
+      for (int i = 0; i < EPT; ++i) {
+        const int e = tid + i * DT;
+        if (e < E) n[e] = rb((x[e] - mean) * rstd * gamma.at(i) + beta.at(i));
+      }
+      for (int e = tid + EPT * DT; e < E; e += DT) n[e] = rb((x[e] - mean) * rstd * ldb(gamma.p, e) + ldb(beta.p, e));
+      __syncthreads();
+      return;
+    }
     float s = 0.0f;
     for (int e = tid; e < E; e += DT) s += x[e];
     const float mean = block_sum(s, shf) * inv_e;
@@ -418,7 +470,8 @@ __global__ void __launch_bounds__(DT, 1) gpt_decode_kernel(const __grid_constant
     prefetch_l2(z.w2, 2ll * E * F);
   };
   auto prefetch_head = [&]() { prefetch_l2(w.head, (long long)E * w.head_ld * 2); };
-#define GRID_BARRIER() do { if (!grid_barrier(p.bar, goal, p.status, &sh_ok)) return; } while (0)
+#define GRID_ARRIVE() grid_arrive(p.bar, goal)
+#define GRID_WAIT() do { if (!grid_wait(p.bar, goal, p.status, &sh_ok)) return; } while (0)
 
   int tok = p.first > 0 ? p.ids_out[p.first - 1] : 0;
   for (int i = p.first; i < p.last; ++i) {
@@ -450,10 +503,11 @@ __global__ void __launch_bounds__(DT, 1) gpt_decode_kernel(const __grid_constant
         norm();
         product(qkv, y.wqkv, slots, red, whole,
                 [&](int, int c, float v) { rows[(long long)pos * ld + c] = __float2bfloat16(v); });
+        GRID_ARRIVE();
         fetch(fused ? out_head : out, y.wo, slots);
         bias.fetch(y.bo, E);
-        GRID_BARRIER();
         if (more) prefetch_layer(l + 1); else prefetch_head();
+        GRID_WAIT();
         if (fused) {
           // few keys: every task of a head works out the head's attention for itself, which costs
           // less than a barrier
@@ -475,7 +529,8 @@ __global__ void __launch_bounds__(DT, 1) gpt_decode_kernel(const __grid_constant
           if (D == 64) attend<64>(rows, ld, E, h, pos, j0, j1, w.scale, red, o);
           else attend<128>(rows, ld, E, h, pos, j0, j1, w.scale, red, o);
         }
-        GRID_BARRIER();
+        GRID_ARRIVE();
+        GRID_WAIT();
         // output projection; each task first puts its heads' splits together
         product(out, y.wo, slots, red,
                 [&](int k0, int len) {
@@ -497,10 +552,11 @@ __global__ void __launch_bounds__(DT, 1) gpt_decode_kernel(const __grid_constant
                 },
                 [&](int s, int c, float v) { p.part[s * E + c] = v; });
         }
+        GRID_ARRIVE();
         fetch(f1, y.w1, slots);
         gamma.fetch(y.ln2_g, E);
         beta.fetch(y.ln2_b, E);
-        GRID_BARRIER();
+        GRID_WAIT();
         add_partials(fused ? p.out_head.ks : p.out.ks);
         norm();
         product(f1, y.w1, slots, red, whole,
@@ -511,8 +567,9 @@ __global__ void __launch_bounds__(DT, 1) gpt_decode_kernel(const __grid_constant
                   asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(v * (k0k1 * (v * v) + k0)));
                   p.h[c] = __float2bfloat16(0.5f * v * t + 0.5f * v);
                 });
+        GRID_ARRIVE();
         fetch(f2, y.w2, slots);
-        GRID_BARRIER();
+        GRID_WAIT();
         product(f2, y.w2, slots, red,
                 [&](int k0, int len) {
                   for (int k = tid * 8; k < len; k += DT * 8) {   // slices start and end at multiples of 8
@@ -525,12 +582,13 @@ __global__ void __launch_bounds__(DT, 1) gpt_decode_kernel(const __grid_constant
                   return xs;
                 },
                 [&](int s, int c, float v) { p.part[s * E + c] = v; });
+        GRID_ARRIVE();
         const GptLayer& z = w.layer[more ? l + 1 : l];
         if (more) fetch(qkv, z.wqkv, slots); else fetch(head, w.head, slots);
         bias.fetch(y.b2, E);
         gamma.fetch(more ? z.ln1_g : w.lnf_g, E);
         beta.fetch(more ? z.ln1_b : w.lnf_b, E);
-        GRID_BARRIER();
+        GRID_WAIT();
       }
       add_partials(p.f2.ks);
     }
@@ -550,8 +608,9 @@ __global__ void __launch_bounds__(DT, 1) gpt_decode_kernel(const __grid_constant
       for (int k = 1; k < WARPS; ++k) kmax = max(kmax, shu[k]);
       p.gmax[blockIdx.x] = kmax;
     }
+    GRID_ARRIVE();
     if (i + 1 < p.last) prefetch_layer(0);
-    GRID_BARRIER();
+    GRID_WAIT();
 
     // ---- sampling, the same in every CTA
     const unsigned short* lg = reinterpret_cast<const unsigned short*>(p.logits);
@@ -559,7 +618,7 @@ __global__ void __launch_bounds__(DT, 1) gpt_decode_kernel(const __grid_constant
     auto count_from = [&](unsigned k0) {
       if (tid == 0) sh_cnt = 0;
       __syncthreads();
-      constexpr int B = 4;                     // loads in flight per thread
+      constexpr int B = 8;                     // loads in flight per thread
       for (int c0 = tid * 8; c0 < V; c0 += B * DT * 8) {
         uint4 q[B];
 #pragma unroll
@@ -698,7 +757,8 @@ __global__ void __launch_bounds__(DT, 1) gpt_decode_kernel(const __grid_constant
     if (blockIdx.x == 0 && tid == 0) p.ids_out[i] = tok;
     __syncthreads();
   }
-#undef GRID_BARRIER
+#undef GRID_ARRIVE
+#undef GRID_WAIT
 }
 
 Split choose_split(int N, int K, int G, int max_ks) {
