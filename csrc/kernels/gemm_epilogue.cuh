@@ -27,7 +27,6 @@ struct KernelParams {
   const __nv_bfloat16* aux_in;
   long long ld_aux;
   int causal_tiles;
-  int causal_k;
   int k_seg;   // GemmArgs::k_seg
   int vec_ok;  // C / residual / aux rows allow 16-byte vector access
   int vec32_ok;  // ... and 32-byte (256-bit) access (bf16 output, residual, aux)

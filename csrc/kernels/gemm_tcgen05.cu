@@ -433,13 +433,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     if (p.causal_tiles == 2) return m0 > n0 + BN - 1;
     return false;
   };
-  // pipeline stages of the k loop for the tile at row m0 (shortened for block-triangular A)
-  auto tile_stages = [&](int m0) -> int {
-    if (!p.causal_k) return num_kb;
-    int k_end = m0 + BM;
-    if (k_end > p.K) k_end = p.K;
-    return (k_end + BK * Cfg::KSUB - 1) / (BK * Cfg::KSUB);
-  };
 
   if (warp_idx == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -454,8 +447,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
         const int n0 = (t / p.tiles_m) * BN;
         if (tile_skipped(m0, n0)) continue;
         const int bi = b % p.batch_inner, bo = b / p.batch_inner;
-        const int nkb = tile_stages(m0);
-        for (int kb = 0; kb < nkb; ++kb) {
+        for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait_bounded(smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag,
                                  &g_gemm_error, 1)) {
             ok = false;
@@ -529,8 +521,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
         }
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        const int nkb = tile_stages(m0);
-        for (int kb = 0; kb < nkb; ++kb) {
+        for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait_bounded(smem_u32(&full_bar[stage]), phase, abort_flag, &g_gemm_error,
                                  3)) {
             ok = false;
@@ -1105,7 +1096,6 @@ KernelParams make_gemm_params(const GemmArgs& a) {
   p.aux_out = (__nv_bfloat16*)a.aux_out;
   p.aux_in = (const __nv_bfloat16*)a.aux_in; p.ld_aux = a.ld_aux;
   p.causal_tiles = a.causal_tiles;
-  p.causal_k = a.causal_k;
   p.k_seg = a.k_seg;
   const int cvec = a.c_fp32 ? 4 : 8;
   bool v = aligned16(a.C) && (a.ldc % cvec == 0) && (a.c_stride_inner % cvec == 0) &&
@@ -1321,7 +1311,7 @@ TileChoice choose_tile(const GemmArgs& a, int K, long long batch, bool c_fp32, b
   struct Cand { int pair, bn; };
   const Cand cands[7] = {{1, 256}, {1, 192}, {1, 128}, {0, 256}, {0, 192}, {0, 128}, {0, 64}};
   const int sms = num_sms();
-  const bool pair_ok = pair_mode() != 0 && a.causal_tiles == 0 && a.causal_k == 0 && a.M > BM;
+  const bool pair_ok = pair_mode() != 0 && a.causal_tiles == 0 && a.M > BM;
   const int force = forced_bn();
   const int clusters = pair_ok ? pair_clusters<256>() : 0;
   TileChoice best;
@@ -1369,7 +1359,7 @@ int choose_split(const GemmArgs& a, TileChoice* slice_tile) {
   TileChoice whole = choose_tile(a, a.K, batch, a.c_fp32 != 0);
   *slice_tile = whole;
   if (batch != 1 || a.act != GEMM_ACT_NONE || a.residual || a.aux_out || a.aux_in ||
-      a.causal_tiles || a.causal_k || a.k_seg || a.K < 2048)
+      a.causal_tiles || a.k_seg || a.K < 2048)
     return 1;
   static const bool no_split = getenv("LT_GEMM_NO_SPLIT") != nullptr;
   if (no_split) return 1;
@@ -1525,7 +1515,7 @@ bool gemm_debug() {
 Route choose_route(const GemmArgs& a, bool have_workspace) {
   const long long batch = (long long)(a.batch_inner < 1 ? 1 : a.batch_inner) * (a.batch_outer < 1 ? 1 : a.batch_outer);
   if ((long long)a.M * a.N * a.K <= 1 << 17) return ROUTE_SIMT;
-  if (!have_workspace || batch > 1 || a.causal_tiles || a.causal_k) return ROUTE_DIRECT;
+  if (!have_workspace || batch > 1 || a.causal_tiles) return ROUTE_DIRECT;
   const double elems = (double)a.M * a.K + (double)a.K * a.N;
   const int parts = a.ab_fp32 ? 3 : 1;
   const double pack = 0.8 * (3.5e-6 + elems * 8.0 / 4.0e12 + choose_tile(a, parts * a.K, 1, a.c_fp32 != 0).cost);
