@@ -7,8 +7,8 @@
 // time against cached keys and values (a full forward per token took 1.8 ms).  A token
 // is a chain of matrix-vector products over all weights (247 MB of bf16 at 124M: 38 us of
 // memory time), so the kernel is built around the chain's latency:
-//   * one CTA per SM; five grid-wide barriers per layer (qkv | attention | out projection | ffn1 |
-//     ffn2), about a microsecond each;
+//   * one CTA per SM; grid-wide barriers of 1.7 us with their skew, four per layer (qkv | attention
+//     and out projection | ffn1 | ffn2) and a fifth between those two when there are many keys;
 //   * every CTA keeps its own copy of the residual stream in shared memory and redoes the cheap
 //     vector work (partial sums, bias, residual, LayerNorm) instead of paying a barrier for it;
 //   * a product [K] x [K, N] is cut into units of 8 columns (16-byte loads), 2 to 16 units per
