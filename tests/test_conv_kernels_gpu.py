@@ -62,3 +62,20 @@ def test_split_k_reduction(M, N, K):
     B.gemm(a, b, a_t=True, out=out, accumulate=True, n_valid=N)
     ad, bd = a.double().t(), b.double()[:, :N]
     assert bool(((out.double() - 1 - ad @ bd).abs() <= K * 2.0 ** -24 * (ad.abs() @ bd.abs() + 1)).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows", [1, 9, 130, 4095, 131072])
+@pytest.mark.parametrize("cols", [4, 8, 16, 32, 64, 128])
+def test_column_sum_does_not_depend_on_the_row_stride(dtype, rows, cols):
+    """Rows that lie back to back and the same rows further apart: the same order of sums."""
+    from luatorch_b200 import _backend as B
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    x = torch.randn(rows, cols, generator=g, device="cuda").to(dtype)
+    wide = torch.zeros(rows, cols + 8, device="cuda", dtype=dtype)
+    wide[:, :cols] = x
+    for acc in (False, True):
+        a, b = torch.full((cols,), 0.5, device="cuda"), torch.full((cols,), 0.5, device="cuda")
+        B.column_sum(x, a, acc)
+        B.column_sum(wide[:, :cols], b, acc)
+        assert torch.equal(a, b)
