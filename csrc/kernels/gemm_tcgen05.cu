@@ -1404,19 +1404,20 @@ cudaError_t launch_choice(const TileChoice& t, const GemmArgs& a, cudaStream_t s
   }
 }
 
-// C = sum_s ws[s] (+ bias) (+ C), four elements per thread.  SG warps share the slices of their
-// elements (warp g adds slices g, g + SG, ...) and the first adds the SG sums: a fixed order.
+// C = sum_s ws[s] (+ bias) (+ C), four elements per thread, slices added in index order.
 // The workspace rows are `ws_ld` floats apart (N rounded up to 4); C is written with 16-byte
 // accesses when `vec` says its rows allow it, element by element otherwise (N = 27 ...).
-// Bound by latency: a convolution's weight gradient has up to 148 slices of a few thousand elements;
-// one thread walking all of them took 11.4 us a call (four in the convolution net), eight 3.7.
-template <int SG>
+// Bound by latency: a convolution's weight gradient has up to 148 slices of a few thousand elements,
+// and one thread walking all of them took 11.4 us a call (four in the convolution net).  STAGED:
+// eight warps bring 64 slices of the block's 32 quads into shared memory, where each element's
+// chain of sums runs in a thread of its own; the next 64 are on their way meanwhile.
+template <bool STAGED>
 __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(const float* __restrict__ ws, int splits, long long slice, int M, int N,
                      int ws_ld, void* C, long long ldc, int c_fp32, int accumulate,
                      const void* __restrict__ bias, int bias_fp32, int vec) {
-  constexpr int QB = 256 / SG;                // quads per block and turn
-  __shared__ float4 sh[SG > 1 ? SG : 1][SG > 1 ? QB : 1];
+  constexpr int QB = STAGED ? 32 : 256;       // quads per block and turn
+  __shared__ float4 sh[STAGED ? 64 : 1][STAGED ? QB : 1];
   pdl_enter();
   const int qpr = ws_ld / 4;
   const long long quads = (long long)M * qpr;
@@ -1425,28 +1426,45 @@ splitk_reduce_kernel(const float* __restrict__ ws, int splits, long long slice, 
     const long long q = q0 + t;
     const long long row = q / qpr;
     const int col = (int)(q - row * qpr) * 4;
-    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (q < quads) {
-      const float* src = ws + row * ws_ld + col;
-      for (int s0 = g; s0 < splits; s0 += 8 * SG) {   // eight loads in flight, added in order
-        float4 v[8];
+    const float* src = ws + row * ws_ld + col;
+    // eight loads in flight; what is past the end is -0, which changes no sum
+    float4 acc = make_float4(-0.0f, -0.0f, -0.0f, -0.0f), v[8];
+    if constexpr (STAGED) {
+      auto load = [&](int s0) {               // warp g: slices s0 + g, s0 + g + 8, ...
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-          v[k] = s0 + k * SG < splits ? *reinterpret_cast<const float4*>(src + (s0 + k * SG) * slice)
-                                      : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int k = 0; k < 8; ++k) {
+          const int s = s0 + g + 8 * k;
+          v[k] = q < quads && s < splits ? *reinterpret_cast<const float4*>(src + s * slice)
+                                         : make_float4(-0.0f, -0.0f, -0.0f, -0.0f);
+        }
+      };
+      load(0);
+      float sum = -0.0f;                      // of element threadIdx.x of the block's 4 x 32
+      for (int s0 = 0; s0 < splits; s0 += 64) {
+        __syncthreads();                      // the slices before have been added
 #pragma unroll
-        for (int k = 0; k < 8; ++k) { acc.x += v[k].x; acc.y += v[k].y; acc.z += v[k].z; acc.w += v[k].w; }
+        for (int k = 0; k < 8; ++k) sh[g + 8 * k][t] = v[k];
+        __syncthreads();
+        if (s0 + 64 < splits) load(s0 + 64);
+        if (threadIdx.x < 4 * QB) {
+          const float* e = reinterpret_cast<const float*>(sh) + threadIdx.x;
+#pragma unroll 16
+          for (int s = 0; s < 64; ++s) sum += e[s * 4 * QB];
+        }
       }
-    }
-    if constexpr (SG > 1) {
-      __syncthreads();                        // the turn before has been read
-      sh[g][t] = acc;
+      __syncthreads();
+      if (threadIdx.x < 4 * QB) reinterpret_cast<float*>(sh)[threadIdx.x] = sum;
       __syncthreads();
       if (g > 0) continue;
+      acc = sh[0][t];
+    } else if (q < quads) {
+      for (int s0 = 0; s0 < splits; s0 += 8) {
 #pragma unroll
-      for (int k = 1; k < SG; ++k) {
-        const float4 v = sh[k][t];
-        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+        for (int k = 0; k < 8; ++k)
+          v[k] = s0 + k < splits ? *reinterpret_cast<const float4*>(src + (s0 + k) * slice)
+                                 : make_float4(-0.0f, -0.0f, -0.0f, -0.0f);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { acc.x += v[k].x; acc.y += v[k].y; acc.z += v[k].z; acc.w += v[k].w; }
       }
     }
     if (q >= quads) continue;
@@ -1607,12 +1625,12 @@ cudaError_t gemm_bf16(const GemmArgs& args, cudaStream_t stream) {
   cudaError_t e = launch_choice(tile, g, stream);
   if (e != cudaSuccess) return e;
   const long long quads = (long long)a.M * (ws_ld / 4);
-  // eight warps per element where there are slices for them and too few elements to fill the chip
-  const bool shared = splits > 8 && quads < 32ll * 8 * num_sms();
-  const int per_block = shared ? 32 : 256;
+  // staged where there are slices for eight warps and too few elements to fill the chip
+  const bool staged = splits > 8 && quads < 32ll * 8 * num_sms();
+  const int per_block = staged ? 32 : 256;
   int blocks = (int)((quads + per_block - 1) / per_block);
   if (blocks > 8 * num_sms()) blocks = 8 * num_sms();
-  cudaError_t re = launch_pdl(shared ? splitk_reduce_kernel<8> : splitk_reduce_kernel<1>, dim3(blocks), dim3(256), 0, stream,
+  cudaError_t re = launch_pdl(staged ? splitk_reduce_kernel<true> : splitk_reduce_kernel<false>, dim3(blocks), dim3(256), 0, stream,
                               (const float*)a.workspace, splits, (long long)a.M * ws_ld, a.M, a.N,
                               ws_ld, a.C, (long long)a.ldc, a.c_fp32, a.accumulate, a.bias,
                               a.bias_fp32, reduce_vec_ok(a) ? 1 : 0);

@@ -79,3 +79,23 @@ def test_column_sum_does_not_depend_on_the_row_stride(dtype, rows, cols):
         B.column_sum(x, a, acc)
         B.column_sum(wide[:, :cols], b, acc)
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("M,N,K", [(32, 27, 131072), (16, 8, 65536), (64, 288, 32768)])
+def test_split_k_slices_are_added_in_index_order(M, N, K):
+    """One product that is not zero per 2048 values of K (so that a slice has at most one), of very
+    different sizes: the result is their fp32 sum from the first to the last."""
+    import numpy as np
+    from luatorch_b200 import _backend as B
+    g = torch.Generator().manual_seed(K)
+    n = K // 2048
+    a, b = torch.zeros(K, M), torch.zeros(K, (N + 7) // 8 * 8)
+    v = (torch.randn(n, M, generator=g) * torch.exp(3 * torch.randn(n, M, generator=g))).bfloat16().float()
+    a[::2048] = v
+    b[::2048] = 1.0
+    out = torch.zeros(M, N, device="cuda")
+    B.gemm(a.cuda().bfloat16(), b.cuda().bfloat16(), a_t=True, out=out, n_valid=N)
+    ref = np.zeros(M, dtype=np.float32)
+    for row in v.numpy():
+        ref = ref + row
+    assert torch.equal(out.cpu(), torch.from_numpy(ref)[:, None].expand(M, N))
