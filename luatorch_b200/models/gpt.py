@@ -89,9 +89,32 @@ class GPT(Module):
         return self.pos_enc(x, seq_len)
 
     # ------------------------------------------------------------------ inference
+    def _is_stock(self) -> bool:
+        """Whether nobody has put code of their own between the layers: every layer is of the type
+        the constructor makes, and no `forward`, `__call__` or `_embed` has been replaced, neither
+        on a class nor on an instance."""
+        if any(c.forward is not f or c.__call__ is not _CALL for c, f in _STOCK.items()):
+            return False
+        if type(self)._embed is not _EMBED or "_embed" in self.__dict__:
+            return False
+        pos = LearnedPE if type(self.pos_enc) is LearnedPE else SinusoidalPE
+        layers = [(self.token_emb, Embedding), (self.pos_enc, pos), (self.emb_drop, Dropout),
+                  (self.final_ln, LayerNorm), (self.head, Linear)]
+        for b in self.blocks:
+            if type(b) is not TransformerBlock:
+                return False
+            layers += [(b, TransformerBlock), (b.ln1, LayerNorm), (b.attn, FlashMultiHeadAttention),
+                       (b.drop1, Dropout), (b.ln2, LayerNorm), (b.ffn1, Linear), (b.ffn2, Linear), (b.drop2, Dropout)]
+            if type(b.attn) is FlashMultiHeadAttention:
+                layers.append((b.attn.out_proj, Linear))
+        for m, c in layers:
+            if type(m) is not c or "forward" in m.__dict__:
+                return False
+        return True
+
     def _inference_weights(self):
         """The bf16 tensors the native inference path reads, or None where it does not apply
-        (CPU, fp32 compute, active dropout, other head sizes, layers of other types)."""
+        (CPU, fp32 compute, active dropout, other head sizes, layers that are not the stock ones)."""
         emb = self.token_emb.weight
         if not emb._t.is_cuda:
             return None
@@ -111,17 +134,13 @@ class GPT(Module):
         out = [view(emb), pos, view(ln.gamma), view(ln.beta), view(head)]
         if self.emb_drop.training and self.emb_drop.p > 0.0 or self.head.use_bias:
             return None
-        if (type(self.token_emb) is not Embedding or type(self.pos_enc) not in (LearnedPE, SinusoidalPE)
-                or type(self.emb_drop) is not Dropout or type(ln) is not LayerNorm or type(self.head) is not Linear):
+        if not self._is_stock():
             return None
         scale = 1.0 / math.sqrt(self.embed_dim // self.num_heads)
         for b in self.blocks:
             a = b.attn
-            if (type(b) is not TransformerBlock or type(a) is not FlashMultiHeadAttention or not a.causal
-                    or a.num_heads != self.num_heads or a.scale != scale
-                    or any(type(m) is not LayerNorm or m.eps != ln.eps for m in (b.ln1, b.ln2))
-                    or any(type(m) is not Linear for m in (a.out_proj, b.ffn1, b.ffn2))
-                    or any(type(m) is not Dropout for m in (b.drop1, b.drop2))
+            if (not a.causal or a.num_heads != self.num_heads or a.scale != scale
+                    or b.ln1.eps != ln.eps or b.ln2.eps != ln.eps
                     or b.training and (b.drop1.p > 0.0 or b.drop2.p > 0.0)
                     or not (a.out_proj.use_bias and b.ffn1.use_bias and b.ffn2.use_bias)):
                 return None
@@ -136,7 +155,7 @@ class GPT(Module):
         """Whether the decode kernel stands for a loop over `forward`: nobody has replaced that
         method, the model fits the kernel's shared memory, the temperature keeps the order of
         the logits, and nobody asked for the checks that follow every launch."""
-        return (getattr(self.forward, "__func__", None) is GPT.forward and not _debug._on
+        return (getattr(self.forward, "__func__", None) is _FORWARD and not _debug._on
                 and 0.0 < temperature < math.inf
                 and B.ext().gpt_decode_fits(self.embed_dim, w[5 + 7].shape[1],
                                             self.embed_dim // self.num_heads, self.vocab_size))
@@ -234,3 +253,10 @@ class GPT(Module):
         return "GPT(vocab=%d, embed=%d, heads=%d, layers=%d, max_seq=%d, params=%d)" % (
             self.vocab_size, self.embed_dim, self.num_heads, self.num_layers, self.max_seq_len,
             self.num_params())
+
+
+# What the native inference path stands for: the methods as they are defined, see GPT._is_stock.
+_CALL = Module.__call__
+_EMBED, _FORWARD = GPT._embed, GPT.forward
+_STOCK = {c: c.forward for c in (Embedding, LearnedPE, SinusoidalPE, Dropout, LayerNorm, Linear,
+                                 FlashMultiHeadAttention, TransformerBlock)}

@@ -128,3 +128,71 @@ def test_context_longer_than_the_model():
     m = _model(97, 64, 1, 1, 24, "learned")
     out = m.generate(list(range(20)), 12, 1.0, 3)
     assert out.shape == [32] and all(0 <= int(t) < 97 for t in out.tolist())
+
+
+def _same_as_layers(m, ids):
+    """The forward without gradients gives what the loop over the layers gives."""
+    import luatorch_b200 as lf
+    with lf.autograd.no_grad():
+        got = m.forward(lf.Tensor.wrap(ids))._t
+    return torch.equal(got, _layerwise(m, ids))
+
+
+LAYERS = {"block": lambda m: m.blocks[1], "attn": lambda m: m.blocks[0].attn, "out_proj": lambda m: m.blocks[1].attn.out_proj,
+          "ln2": lambda m: m.blocks[0].ln2, "ffn1": lambda m: m.blocks[1].ffn1, "ffn2": lambda m: m.blocks[0].ffn2,
+          "emb_drop": lambda m: m.emb_drop, "final_ln": lambda m: m.final_ln,
+          "head": lambda m: m.head}
+
+
+@pytest.mark.parametrize("where", ["instance", "class"])
+@pytest.mark.parametrize("layer", list(LAYERS))
+def test_a_replaced_forward_is_called(layer, where, monkeypatch):
+    """Scoring and sampling call what a program has put in a layer's place."""
+    import luatorch_b200 as lf
+    m = _model(97, 128, 2, 2, 24, "learned")
+    ids = torch.arange(5, device="cuda", dtype=torch.int32).reshape(1, 5)
+    target = LAYERS[layer](m)
+    stock, seen = target.forward, []
+
+    def doubled(*args, **kwargs):
+        seen.append(1)
+        if where == "class":
+            out = original(*args, **kwargs)
+        else:
+            out = stock(*args, **kwargs)
+        return lf.Tensor(_data=out._t * 2)
+
+    if where == "class":
+        owner = next(c for c in type(target).__mro__ if "forward" in vars(c))
+        original = owner.forward
+        monkeypatch.setattr(owner, "forward", doubled)
+    else:
+        target.forward = doubled
+    assert _same_as_layers(m, ids) and seen
+    seen.clear()
+    assert m.generate([1, 2, 3], 3, 1.0, 5).shape == [6] and len(seen) >= 3
+
+
+def test_a_replaced_call_or_embedding_is_called(monkeypatch):
+    import luatorch_b200 as lf
+    seen = []
+
+    class Shifted(lf.models.GPT):
+        def _embed(self, ids, seq_len):
+            seen.append(seq_len)
+            return super()._embed((ids.int() + 1) % 97, seq_len)
+
+    lf.manual_seed(2)
+    m = Shifted(97, 128, 2, 1, 24, 0.0)
+    lf.cuda.amp.autocast_bf16(m)
+    m.eval()
+    ids = torch.arange(5, device="cuda", dtype=torch.int32).reshape(1, 5)
+    assert _same_as_layers(m, ids) and len(seen) == 2
+    m = _model(97, 128, 2, 1, 24, "learned")
+    call = lf.nn.Module.__call__
+    monkeypatch.setattr(lf.nn.Module, "__call__", lambda self, *a, **k: (seen.append(type(self)), call(self, *a, **k))[1])
+    seen.clear()
+    assert _same_as_layers(m, ids) and lf.nn.Linear in seen
+    seen.clear()
+    m.generate([1, 2, 3], 2, 1.0, 5)
+    assert lf.nn.LayerNorm in seen
