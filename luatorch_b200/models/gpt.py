@@ -115,6 +115,8 @@ class GPT(Module):
     def _inference_weights(self):
         """The bf16 tensors the native inference path reads, or None where it does not apply
         (CPU, fp32 compute, active dropout, other head sizes, layers that are not the stock ones)."""
+        if not self._is_stock():      # first: layers of other types have other attributes
+            return None
         emb = self.token_emb.weight
         if not emb._t.is_cuda:
             return None
@@ -133,8 +135,6 @@ class GPT(Module):
         ln = self.final_ln
         out = [view(emb), pos, view(ln.gamma), view(ln.beta), view(head)]
         if self.emb_drop.training and self.emb_drop.p > 0.0 or self.head.use_bias:
-            return None
-        if not self._is_stock():
             return None
         scale = 1.0 / math.sqrt(self.embed_dim // self.num_heads)
         for b in self.blocks:

@@ -196,3 +196,32 @@ def test_a_replaced_call_or_embedding_is_called(monkeypatch):
     seen.clear()
     m.generate([1, 2, 3], 2, 1.0, 5)
     assert lf.nn.LayerNorm in seen
+
+
+@pytest.mark.parametrize("what", ["head", "final_ln", "pos_enc", "emb_drop", "block", "attn"])
+def test_layers_of_other_types(what):
+    """A module of the program's own in a layer's place: the loop over the layers, whatever it has inside."""
+    import luatorch_b200 as lf
+    nn = lf.nn
+
+    class Own(nn.Module):                       # has none of the stock layers' attributes
+        def __init__(self, fn):
+            self.fn = fn
+
+        def forward(self, x, *args, **kwargs):
+            return self.fn(x, *args, **kwargs)
+
+    m = _model(97, 128, 2, 2, 24, "sinusoidal")
+    if what == "block":
+        m.blocks[1] = Own(lambda x, s: x)
+    elif what == "attn":
+        m.blocks[0].attn = Own(lambda x, seq_len=None, residual=None: residual)
+    elif what == "pos_enc":
+        stock = _model(97, 128, 2, 2, 24, "sinusoidal")
+        m.pos_enc, m._embed = Own(None), stock._embed
+    else:
+        stock = getattr(m, what)
+        setattr(m, what, Own(lambda x: stock(x)))
+    ids = torch.arange(5, device="cuda", dtype=torch.int32).reshape(1, 5)
+    assert _same_as_layers(m, ids)
+    assert m.generate([1, 2, 3], 3, 1.0, 5).shape == [6]
