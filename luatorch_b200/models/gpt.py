@@ -149,6 +149,11 @@ class GPT(Module):
                     view(b.ffn1.bias), view(b.ffn2.weight), view(b.ffn2.bias)]
         if len(self.blocks) > 96 or any(t is None for t in out) or out[4].shape[1] % 8:
             return None
+        # every block alike: the kernels take one set of widths
+        E, F = self.embed_dim, self.blocks[0].ffn1.out_features
+        widths = [(E,), (E,), (E, 3 * E), (E, E), (E,), (E,), (E,), (E, F), (F,), (F, E), (E,)]
+        if F % 8 or [t.shape for t in out[5:]] != widths * len(self.blocks):
+            return None
         return out
 
     def _decode_applies(self, w, temperature) -> bool:

@@ -225,3 +225,28 @@ def test_layers_of_other_types(what):
     ids = torch.arange(5, device="cuda", dtype=torch.int32).reshape(1, 5)
     assert _same_as_layers(m, ids)
     assert m.generate([1, 2, 3], 3, 1.0, 5).shape == [6]
+
+
+@pytest.mark.parametrize("widths", [(4, 2), (2, 4), (1, 3)])
+def test_blocks_of_different_width(widths):
+    import luatorch_b200 as lf
+    lf.manual_seed(4)
+    m = lf.models.GPT(97, 128, 2, 2, 24, 0.0, pos="learned")
+    m.blocks = [lf.nn.TransformerBlock(128, 2, 0.0, w) for w in widths]
+    lf.cuda.amp.autocast_bf16(m)
+    m.eval()
+    ids = torch.arange(5, device="cuda", dtype=torch.int32).reshape(1, 5)
+    assert _same_as_layers(m, ids)
+    assert m.generate([1, 2, 3], 3, 1.0, 5).shape == [6]
+
+
+def test_feed_forward_width_that_is_no_multiple_of_eight():
+    import luatorch_b200 as lf
+    lf.manual_seed(4)
+    m = lf.models.GPT(97, 128, 2, 1, 24, 0.0, pos="learned")
+    m.blocks[0].ffn1, m.blocks[0].ffn2 = lf.nn.Linear(128, 100), lf.nn.Linear(100, 128)
+    lf.cuda.amp.autocast_bf16(m)
+    m.eval()
+    ids = torch.arange(5, device="cuda", dtype=torch.int32).reshape(1, 5)
+    assert _same_as_layers(m, ids)
+    assert m.generate([1, 2, 3], 3, 1.0, 5).shape == [6]
