@@ -147,7 +147,7 @@ class GPT(Module):
             out += [view(b.ln1.gamma), view(b.ln1.beta), view(a.qkv_weight), view(a.out_proj.weight),
                     view(a.out_proj.bias), view(b.ln2.gamma), view(b.ln2.beta), view(b.ffn1.weight),
                     view(b.ffn1.bias), view(b.ffn2.weight), view(b.ffn2.bias)]
-        if len(self.blocks) > 96 or any(t is None for t in out) or out[4].shape[1] % 8:
+        if not 0 < len(self.blocks) <= 96 or any(t is None for t in out) or out[4].shape[1] % 8:
             return None
         # every block alike: the kernels take one set of widths
         E, F = self.embed_dim, self.blocks[0].ffn1.out_features

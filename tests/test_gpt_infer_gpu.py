@@ -250,3 +250,11 @@ def test_feed_forward_width_that_is_no_multiple_of_eight():
     ids = torch.arange(5, device="cuda", dtype=torch.int32).reshape(1, 5)
     assert _same_as_layers(m, ids)
     assert m.generate([1, 2, 3], 3, 1.0, 5).shape == [6]
+
+
+def test_a_model_without_blocks():
+    import luatorch_b200 as lf
+    m = _model(97, 128, 2, 0, 24, "learned")
+    ids = torch.arange(5, device="cuda", dtype=torch.int32).reshape(1, 5)
+    assert _same_as_layers(m, ids)
+    assert m.generate([1, 2, 3], 3, 1.0, 5).shape == [6]
