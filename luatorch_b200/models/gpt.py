@@ -149,8 +149,11 @@ class GPT(Module):
                     view(b.ffn1.bias), view(b.ffn2.weight), view(b.ffn2.bias)]
         if not 0 < len(self.blocks) <= 96 or any(t is None for t in out) or out[4].shape[1] % 8:
             return None
-        # every block alike: the kernels take one set of widths
+        # every block alike: the kernels take one set of widths, and vocab_size for table and head
         E, F = self.embed_dim, self.blocks[0].ffn1.out_features
+        if (out[0].shape != (self.vocab_size, E) or out[1].shape[1:] != (E,) or out[2].shape != (E,)
+                or out[3].shape != (E,) or self.head.out_features != self.vocab_size or out[4].shape[0] != E):
+            return None
         widths = [(E,), (E,), (E, 3 * E), (E, E), (E,), (E,), (E,), (E, F), (F,), (F, E), (E,)]
         if F % 8 or [t.shape for t in out[5:]] != widths * len(self.blocks):
             return None

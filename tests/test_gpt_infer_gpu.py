@@ -258,3 +258,19 @@ def test_a_model_without_blocks():
     ids = torch.arange(5, device="cuda", dtype=torch.int32).reshape(1, 5)
     assert _same_as_layers(m, ids)
     assert m.generate([1, 2, 3], 3, 1.0, 5).shape == [6]
+
+
+def test_table_and_head_of_other_widths():
+    """An embedding with more rows than `vocab_size`, a head with fewer or more columns."""
+    import luatorch_b200 as lf
+    for rows, cols in ((120, 97), (97, 40), (97, 128)):
+        lf.manual_seed(4)
+        m = lf.models.GPT(97, 128, 2, 1, 24, 0.0, pos="learned")
+        m.token_emb, m.head = lf.nn.Embedding(rows, 128), lf.nn.Linear(128, cols, False, pad_out=True)
+        lf.cuda.amp.autocast_bf16(m)
+        m.eval()
+        ids = torch.tensor([[0, 5, rows - 1, 7]], device="cuda", dtype=torch.int32)
+        with lf.autograd.no_grad():
+            assert m.forward(lf.Tensor.wrap(ids)).shape == [4, cols]
+        assert _same_as_layers(m, ids)
+        assert m.generate([1, 2, 3], 3, 1.0, 5).shape == [6]
