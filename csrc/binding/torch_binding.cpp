@@ -775,6 +775,8 @@ Tensor gpt_generate(const std::vector<Tensor>& w, int64_t heads, int64_t vocab, 
   const lt::GptWeights g = gpt_weights(w, heads, vocab, eps);
   const int64_t S = ids.numel(), n = rnd.numel(), rows = S + n - 1;
   TORCH_CHECK(S > 0 && n > 0 && rows <= w[1].size(0), "gpt_generate: sequence too long");
+  for (const Tensor& t : w)   // the decode kernel reads its matrices in 16-byte words
+    TORCH_CHECK(reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, "gpt_generate: weights must start on 16 bytes");
   Tensor ws = bytes_like(ids, lt::gpt_forward_workspace(g, S));
   Tensor cache = at::empty({g.layers, rows, 3 * g.embed}, w[0].options());
   Tensor scratch = bytes_like(ids, lt::gpt_decode_scratch(g));

@@ -161,10 +161,11 @@ class GPT(Module):
 
     def _decode_applies(self, w, temperature) -> bool:
         """Whether the decode kernel stands for a loop over `forward`: nobody has replaced that
-        method, the model fits the kernel's shared memory, the temperature keeps the order of
-        the logits, and nobody asked for the checks that follow every launch."""
+        method, the model fits the kernel's shared memory, its weights allow 16-byte loads, the
+        temperature keeps the order of the logits, and nobody asked for the checks that follow every launch."""
         return (getattr(self.forward, "__func__", None) is _FORWARD and not _debug._on
                 and 0.0 < temperature < math.inf
+                and all(t.data_ptr() % 16 == 0 for t in w)
                 and B.ext().gpt_decode_fits(self.embed_dim, w[5 + 7].shape[1],
                                             self.embed_dim // self.num_heads, self.vocab_size))
 

@@ -274,3 +274,23 @@ def test_table_and_head_of_other_widths():
             assert m.forward(lf.Tensor.wrap(ids)).shape == [4, cols]
         assert _same_as_layers(m, ids)
         assert m.generate([1, 2, 3], 3, 1.0, 5).shape == [6]
+
+
+@pytest.mark.parametrize("name", ["ffn1", "ffn2", "out_proj", "qkv"])
+def test_weights_off_the_16_byte_grid(name):
+    """bf16 weights that are a view at an odd offset: the decode kernel's 16-byte loads cannot take them."""
+    import luatorch_b200 as lf
+    from luatorch_b200 import _C
+    m = _model(97, 128, 2, 2, 24, "learned")
+    b = m.blocks[1]
+    p = {"ffn1": b.ffn1.weight, "ffn2": b.ffn2.weight, "out_proj": b.attn.out_proj.weight, "qkv": b.attn.qkv_weight}[name]
+    t = p._compute
+    buf = torch.empty(t.numel() + 1, device="cuda", dtype=t.dtype)
+    p._compute = buf[1:].view(t.shape).copy_(t)
+    w = m._inference_weights()
+    assert w is not None and not m._decode_applies(w, 1.0)
+    with pytest.raises(RuntimeError, match="16 bytes"):
+        _C.gpt_generate(w, 2, 97, 1e-5, torch.zeros(3, device="cuda", dtype=torch.int32), torch.rand(2, device="cuda"), 1.0, 5)
+    ids = torch.arange(5, device="cuda", dtype=torch.int32).reshape(1, 5)
+    assert _same_as_layers(m, ids)
+    assert m.generate([1, 2, 3], 3, 1.0, 5).shape == [6]
