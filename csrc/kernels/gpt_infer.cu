@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(DT, 1) gpt_decode_kernel(const __grid_constant
   float* xs = n + E;                         // activations of a product
   float* red = xs + (E > F ? E : F);
   __shared__ float2 sh[32];
-  __shared__ int sh_ok, sh_cnt;
+  __shared__ int sh_ok, sh_cnt, sh_last;
   __shared__ unsigned sh_key;
   __shared__ unsigned cand[MAX_CAND];        // keys of the logits above the bound
   __shared__ int cand_at[MAX_CAND];          // and their places
@@ -732,24 +732,33 @@ __global__ void __launch_bounds__(DT, 1) gpt_decode_kernel(const __grid_constant
     }
     __syncthreads();                           // shu has been read
     if (lane == 31) shf[warp] = incl;
-    if (tid == 0) sh_cnt = V - 1;
+    if (tid == 0) { sh_cnt = V - 1; sh_last = -1; }
     __syncthreads();
     float before = 0.0f, total = 0.0f;
     for (int k = 0; k < WARPS; ++k) {
       if (k < warp) before += shf[k];
       total += shf[k];
     }
+    // only threads with weight may draw; the last of them stands in where rounding (a scan's prefixes
+    // depend on the place) leaves none that reaches the goal
+    const int last = __reduce_max_sync(0xffffffffu, mine > 0.0f ? tid : -1);
+    if (lane == 0) atomicMax(&sh_last, last);
+    __syncthreads();
     const float goal_w = p.rnd[i] * total;
-    if (before + incl >= goal_w && c0 < c1) {  // the first such thread holds the token: min over all
+    if (mine > 0.0f && (before + incl >= goal_w || tid == sh_last)) {   // the first such thread: min over all
       if (few) {
         atomicMin(&sh_cnt, at[tid]);
       } else {
         float run = before + incl - mine;
+        int pick = V - 1;                      // a column that the cut has left
         for (int c = c0; c < c1; ++c) {
           const unsigned k = key_of(lg[c]);
-          if (k >= thresh) run += weight(k);
-          if (run >= goal_w || c + 1 == c1) { atomicMin(&sh_cnt, c); break; }
+          if (k < thresh) continue;
+          pick = c;
+          run += weight(k);
+          if (run >= goal_w) break;
         }
+        atomicMin(&sh_cnt, pick);
       }
     }
     __syncthreads();

@@ -83,6 +83,8 @@ def test_decode_draws_from_the_layers_distribution(vocab, embed, heads, layers, 
         t = toks[prompt + i]
         lo = float(cdf[t - 1]) if t else 0.0
         assert lo - 0.04 <= rnd[i] <= float(cdf[t]) + 0.04, (i, t, lo, rnd[i], float(cdf[t]))
+        if 0 < top_k < vocab:       # and it is among the top_k: two logits, two ulps of 2^-4 each
+            assert float(logits[i][t]) >= float(torch.topk(logits[i], top_k).values[-1]) - 0.25 / temperature
 
 
 def test_decode_kernel_only_stands_for_the_stock_loop():
@@ -294,3 +296,57 @@ def test_weights_off_the_16_byte_grid(name):
     ids = torch.arange(5, device="cuda", dtype=torch.int32).reshape(1, 5)
     assert _same_as_layers(m, ids)
     assert m.generate([1, 2, 3], 3, 1.0, 5).shape == [6]
+
+
+def _exact_model(vocab, embed):
+    """One block that adds nothing, embeddings of +-1 that LayerNorm leaves as they are, a head of
+    multiples of 1/16: every logit is exact in fp32 whatever the order of the sums."""
+    import luatorch_b200 as lf
+    lf.manual_seed(1)
+    m = lf.models.GPT(vocab, embed, embed // 64, 1, 64, 0.0, pos="learned")
+    g = torch.Generator().manual_seed(vocab)
+    m.pos_enc.weight._t.zero_()
+    for lin in (m.blocks[0].attn.out_proj, m.blocks[0].ffn2):
+        lin.weight._t.zero_()
+    signs = torch.ones(embed)
+    signs[:embed // 2] = -1
+    order = torch.rand(vocab, embed, generator=g).argsort(1)
+    m.token_emb.weight._t.copy_(signs[order])
+    m.head.weight._t.copy_(torch.randint(-6, 7, (embed, vocab), generator=g) / 16.0)
+    lf.cuda.amp.autocast_bf16(m)
+    return m.eval()
+
+
+@pytest.mark.parametrize("embed", [64, 128])           # 64: no room for a list of candidates
+@pytest.mark.parametrize("vocab,top_k", [
+    (777, 5), (777, 140),          # few candidates
+    (2500, 148),                   # ties at the cut
+    (777, 300), (9000, 5000),      # the threshold by bisection, runs of columns per thread
+    (777, 0), (9000, 0), (50257, 0),
+])
+def test_decode_draws_the_exact_token(vocab, top_k, embed):
+    """Known logits: the token is the one at the uniform number under their distribution, and a
+    column that the cut has removed is never drawn, at the ends of the range of rnd either."""
+    from luatorch_b200 import _C
+    m = _exact_model(vocab, embed)
+    w = m._inference_weights()
+    assert m._decode_applies(w, 1.0)
+    g = torch.Generator().manual_seed(7)
+    rnd = torch.rand(30, generator=g)
+    rnd[::5] = 0.0
+    rnd[1::5] = 1 - 2.0 ** -24
+    toks = [3] + _C.gpt_generate(w, embed // 64, vocab, m.final_ln.eps, torch.tensor([3], device="cuda", dtype=torch.int32),
+                                 rnd.cuda(), 1.0, top_k).tolist()[:-1]
+    logits = _layerwise(m, torch.tensor([toks], dtype=torch.int32, device="cuda"))[:-1].double().cpu()
+    for i in range(30):
+        v = logits[i]
+        if top_k:
+            v = torch.where(v < torch.topk(v, top_k).values[-1], torch.full_like(v, -float("inf")), v)
+        p = torch.softmax(v, 0)
+        cdf, t, r = torch.cumsum(p, 0), toks[i + 1], float(rnd[i])
+        assert float(p[t]) > 0.0, (i, t)
+        # fp32 sums of at most 50257 weights, expf to a few ulps: far below 1e-4 of the total
+        lo = float(cdf[t] - p[t])
+        assert lo - 1e-4 <= r <= float(cdf[t]) + 1e-4, (i, t, lo, r, float(cdf[t]))
+        if abs(lo - r) > 1e-4 and abs(float(cdf[t]) - r) > 1e-4:
+            assert t == int(torch.searchsorted(cdf, torch.tensor(r, dtype=torch.float64)))
