@@ -98,6 +98,20 @@ struct GemmGather {
 // Bytes of workspace that `args` would use (0: none).
 size_t gemm_workspace_bytes(const GemmArgs& args);
 
+// What a product does with GemmArgs::workspace.  Its last kernel reads it: the split-K reduction the
+// partial sums, the packed product its operands.  The caller may free the workspace on return, and
+// the allocator may hand the same memory to the next product at once; that one may then not
+// write before this one has finished.
+enum GemmWorkspaceUse { GEMM_WS_NONE, GEMM_WS_SPLIT_K, GEMM_WS_PACKED };
+// GemmArgs::overlap_prev that a product with this use may keep.  `prev_reads`: whether the product
+// launched last reads its workspace; updated.
+inline int gemm_overlap_allowed(bool& prev_reads, GemmWorkspaceUse use, int overlap_prev) {
+  // the packed product follows its own packing launch, which its caller knows nothing of
+  if (use == GEMM_WS_PACKED || (use == GEMM_WS_SPLIT_K && prev_reads)) overlap_prev = 0;
+  prev_reads = use != GEMM_WS_NONE;
+  return overlap_prev;
+}
+
 // Returns cudaSuccess or the launch error.  Operands that satisfy TMA alignment (bf16, base 16 B
 // aligned, lda/ldb multiples of 8 elements) take the TMA kernels; others are loaded by the
 // direct kernel, or packed into the workspace first where the product is large enough to repay

@@ -1553,8 +1553,7 @@ size_t gemm_workspace_bytes(const GemmArgs& a) {
   return s > 1 ? (size_t)s * (size_t)a.M * (size_t)ws_ld_of(a) * sizeof(float) : 0;
 }
 
-// True while the kernel launched last by gemm_bf16 is a split-K reduction (it reads the
-// workspace): a split-K GEMM that follows may then not start before that kernel has finished.
+// Whether the kernel launched last by gemm_bf16 reads the workspace, see gemm_overlap_allowed().
 static thread_local bool g_prev_reads_workspace = false;
 
 cudaError_t gemm_bf16(const GemmArgs& args, cudaStream_t stream) {
@@ -1575,9 +1574,11 @@ cudaError_t gemm_bf16(const GemmArgs& args, cudaStream_t stream) {
     return launch_choice(t, a, stream);
   }
   if (!gemm_uses_tensor_cores(a)) {
-    g_prev_reads_workspace = false;
     const bool ws = a.workspace && a.workspace_bytes >= gemm_pack_bytes(a);
-    switch (choose_route(a, ws)) {
+    const Route route = choose_route(a, ws);
+    a.overlap_prev = gemm_overlap_allowed(g_prev_reads_workspace, route == ROUTE_PACK ? GEMM_WS_PACKED : GEMM_WS_NONE,
+                                          a.overlap_prev);
+    switch (route) {
       case ROUTE_SIMT: return launch_simt(a, stream);
       case ROUTE_DIRECT: return gemm_direct(a, stream);
       case ROUTE_PACK: break;
@@ -1585,7 +1586,6 @@ cudaError_t gemm_bf16(const GemmArgs& args, cudaStream_t stream) {
     const cudaError_t e = gemm_pack(a, a.workspace, stream);
     if (e != cudaSuccess) return e;
     a.workspace = nullptr;
-    a.overlap_prev = 0;
     return launch_choice(choose_tile(a, a.K, 1, a.c_fp32 != 0), a, stream);
   }
   TileChoice tile;
@@ -1598,13 +1598,9 @@ cudaError_t gemm_bf16(const GemmArgs& args, cudaStream_t stream) {
   if (gemm_debug())
     fprintf(stderr, "gemm %dx%dx%d -> %s BN=%d split %d (model %.1f us)\n", a.M, a.N, a.K,
             tile.pair ? "pair" : "single", tile.bn, splits, tile.cost * 1e6);
-  if (splits == 1) {
-    g_prev_reads_workspace = false;
-    return launch_choice(tile, a, stream);
-  }
+  a.overlap_prev = gemm_overlap_allowed(g_prev_reads_workspace, splits > 1 ? GEMM_WS_SPLIT_K : GEMM_WS_NONE, a.overlap_prev);
+  if (splits == 1) return launch_choice(tile, a, stream);
   // K slices as batches into the fp32 workspace, then one deterministic reduction
-  if (g_prev_reads_workspace) a.overlap_prev = 0;
-  g_prev_reads_workspace = true;
   GemmArgs g = a;
   const int ks = a.K / splits;
   g.K = ks;

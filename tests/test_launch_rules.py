@@ -29,3 +29,15 @@ def test_late_wait_rules_host_program():
         assert r.returncode == 0, r.stderr[-3000:]
         r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
         assert r.returncode == 0 and "RULES_OK" in r.stdout, (r.stdout, r.stderr)
+
+
+@pytest.mark.skipif(_nvcc() is None, reason="nvcc not found")
+def test_workspace_rules_host_program(tmp_path):
+    """Which product may start in the tail of one that reads its workspace (csrc/kernels/gemm.h)."""
+    exe = str(tmp_path / "workspace_rules")
+    r = subprocess.run([_nvcc(), "-std=c++17", "-O1", "-I", os.path.join(ROOT, "csrc", "kernels"),
+                        os.path.join(ROOT, "tests", "cpp", "workspace_rules.cu"), "-o", exe],
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-3000:]
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0 and "RULES_OK" in r.stdout, (r.stdout, r.stderr)
