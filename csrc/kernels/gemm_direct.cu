@@ -181,9 +181,10 @@ gemm_direct_kernel(const DirectParams d, const KernelParams p) {
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int S = d.splits;
   const int rank = S > 1 ? (int)cluster_cta_rank() : 0;
-  const int tile = (int)blockIdx.x / S;
+  // one grid dimension for clusters, tiles and batch: the others end at 65535
+  const int tiles = p.tiles_m * p.tiles_n, unit = (int)(blockIdx.x / S), b = unit / tiles, tile = unit % tiles;
   const int m0 = (tile % p.tiles_m) * BM, n0 = (tile / p.tiles_m) * BN;
-  const int bi = (int)blockIdx.z % p.batch_inner, bo = (int)blockIdx.z / p.batch_inner;
+  const int bi = b % p.batch_inner, bo = b / p.batch_inner;
   const int steps = (p.K + BK - 1) / BK;
   const int it0 = (int)((long long)steps * rank / S), it1 = (int)((long long)steps * (rank + 1) / S);
 
@@ -389,7 +390,7 @@ cudaError_t launch(const DirectParams& d, const KernelParams& p, cudaStream_t st
   auto* kernel = gemm_direct_kernel<BN, T, SPLIT, A_MN, B_MN>;
   static const cudaError_t attr = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
   if (attr != cudaSuccess) return attr;
-  const dim3 grid((unsigned)(p.tiles_m * p.tiles_n * d.splits), 1, (unsigned)p.batch_total);
+  const dim3 grid((unsigned)((long long)p.tiles_m * p.tiles_n * d.splits * p.batch_total));
   const cudaError_t e = launch_pdl_cluster(kernel, grid, dim3(THREADS), C::SMEM, stream, d.splits, d, p);
   if (e != cudaSuccess) return e;
   g_gemm_launches.fetch_add(1, std::memory_order_relaxed);

@@ -985,13 +985,14 @@ gemm_simt_kernel(const E* __restrict__ A, const E* __restrict__ B,
   constexpr int T = 32, KT = 32;
   __shared__ float sa[KT][T + 1];
   __shared__ float sb[KT][T + 1];
-  const int b = blockIdx.z;
+  // one grid dimension for tiles and batch: the others end at 65535
+  const int tiles = p.tiles_m * p.tiles_n, b = (int)(blockIdx.x / tiles), tile = (int)(blockIdx.x % tiles);
   const int bi = b % p.batch_inner, bo = b / p.batch_inner;
   A += bi * a_stride_inner + bo * a_stride_outer;
   B += bi * b_stride_inner + bo * b_stride_outer;
   const size_t esz = p.c_fp32 ? 4 : 2;
   char* c_base = (char*)p.C + (size_t)(bi * p.c_stride_inner + bo * p.c_stride_outer) * esz;
-  const int m0 = blockIdx.y * T, n0 = blockIdx.x * T;
+  const int m0 = tile / p.tiles_n * T, n0 = tile % p.tiles_n * T;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // 16 x 16 threads, 2x2 outputs each
   float acc[2][2] = {{0, 0}, {0, 0}};
   for (int k0 = 0; k0 < p.K; k0 += KT) {
@@ -1265,7 +1266,9 @@ cudaError_t launch_simt(const GemmArgs& a, cudaStream_t stream) {
   p.vec_ok = 0;
   long long a_sm = a.a_mn_major ? 1 : a.lda, a_sk = a.a_mn_major ? a.lda : 1;
   long long b_sk = a.b_mn_major ? a.ldb : 1, b_sn = a.b_mn_major ? 1 : a.ldb;
-  dim3 grid((a.N + 31) / 32, (a.M + 31) / 32, p.batch_total);
+  p.tiles_m = (a.M + 31) / 32;
+  p.tiles_n = (a.N + 31) / 32;
+  const dim3 grid((unsigned)((long long)p.tiles_m * p.tiles_n * p.batch_total));
   if (a.ab_fp32)
     gemm_simt_kernel<float><<<grid, 256, 0, stream>>>(
         (const float*)a.A, (const float*)a.B, a_sm, a_sk, b_sk, b_sn,

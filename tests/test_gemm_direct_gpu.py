@@ -66,3 +66,16 @@ def test_batched_fp32():
     out = B.bmm(a, b)
     for i in range(5):
         _check(out[i], a[i], b[i], torch.float32)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("M,N,K", [(3, 5, 4), (1, 2, 200), (64, 33, 64)])
+def test_more_matrices_than_a_grid_dimension_holds(M, N, K, dtype):
+    from luatorch_b200 import _C, _backend as B
+    g = torch.Generator(device="cuda").manual_seed(7)
+    n = 65600
+    a, b = torch.randn(n, M, K, generator=g, device="cuda").to(dtype), torch.randn(n, K, N, generator=g, device="cuda").to(dtype)
+    out = B.bmm(a, b)
+    for i in (0, 1, 32767, 65535, 65536, n - 1):
+        _check(out[i], a[i], b[i], dtype)
+    assert _C.gemm_device_error() == 0
