@@ -74,8 +74,8 @@ attn_stats_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
                   long long do_sb, long long do_ss, long long do_sh) {
   pdl_enter();
   constexpr int PARTS = D / 64;              // 16-byte loads per lane: 8 lanes per query
-  const int h = blockIdx.x, b = blockIdx.y;
-  const int s = (int)blockIdx.z * STAT_ROWS + (threadIdx.x >> 3), v = threadIdx.x & 7;
+  const int h = blockIdx.x % H, b = blockIdx.y;   // tiles in x: the other dimensions end at 65535
+  const int s = (int)(blockIdx.x / H) * STAT_ROWS + (threadIdx.x >> 3), v = threadIdx.x & 7;
   float t[PARTS][4] = {};
   if (s < S) {
     const __nv_bfloat16* op = o + b * o_sb + s * o_ss + h * o_sh + v * 8;
@@ -529,7 +529,7 @@ cudaError_t flash_attention_backward(const AttnArgs& a, const AttnBwdArgs& g, cu
     return cudaErrorInvalidValue;
 
   const auto stats = a.D == 64 ? attn_stats_kernel<64> : attn_stats_kernel<128>;
-  cudaError_t e = launch_pdl(stats, dim3(a.H, a.B, Sp / STAT_ROWS), dim3(STAT_ROWS * 8), 0, stream,
+  cudaError_t e = launch_pdl(stats, dim3((unsigned)a.H * (Sp / STAT_ROWS), a.B), dim3(STAT_ROWS * 8), 0, stream,
                              (const __nv_bfloat16*)a.o, (const __nv_bfloat16*)g.d_o, (const float*)a.lse, lse2,
                              dsc, a.H, a.S, Sp, a.scale, (long long)a.o_sb, (long long)a.o_ss, (long long)a.o_sh,
                              (long long)g.do_sb, (long long)g.do_ss, (long long)g.do_sh);
