@@ -53,7 +53,7 @@ struct GemmArgs {
   int64_t ld_aux = 0;
   int causal_tiles = 0;  // 1: skip output tiles strictly above the diagonal (n0 > m0 + BM - 1);
                          // 2: skip tiles strictly below (m0 > n0 + BN - 1)
-  // k_seg > 0: both operands hold TWO matrices of k_seg (a multiple of 128) along k, the hi and lo
+  // k_seg > 0: both operands hold TWO matrices of k_seg (a multiple of 64) along k, the hi and lo
   // parts of fp32 values, and K = 3 k_seg runs over hi*hi, hi*lo and lo*hi.
   int k_seg = 0;
   // n > 0: this product reads nothing that the n kernels launched just before it on `stream`

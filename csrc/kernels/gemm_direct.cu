@@ -430,15 +430,17 @@ double gemm_direct_cost(const GemmArgs& a) {
 
 // ------------------------------------------------------------------------------ packing
 // Copies of the operands that TMA can address.  K-major [R, K] becomes [R, parts x Kp] and MN-major
-// [K, C] becomes [parts x Kp, Cp], Kp a multiple of 128, Cp of 8; parts = 2 for fp32 (hi, lo), 1 for
-// bf16.  Rows and columns of k beyond K are zero.  One launch for both operands; a thread makes
-// eight values (16-byte stores), a block 2048 of one operand.
+// [K, C] becomes [parts x Kp, Cp], Kp a multiple of 64, Cp of 8; parts = 2 for fp32 (hi, lo), 1 for
+// bf16.  Rows and columns of k beyond K are zero; the matrices of a batch follow one another.  One launch
+// for both operands; a thread makes eight values (16-byte stores), a block 2048 of one matrix.
 namespace {
 
 struct PackOperand {
   const void* src;
   __nv_bfloat16* dst;
   long long ld, dst_ld, lo;    // lo: distance of the lo part in elements
+  long long si, so, dst_matrix;  // batch strides of the source, elements of a copied matrix
+  int batch_inner, blocks;     // blocks of one matrix
   int rows, cols;              // of the source
   int drows, dcols;            // of one part
 };
@@ -466,13 +468,15 @@ __device__ __forceinline__ uint4 load16_any(const void* s) {
 }
 
 template <typename T>
-__device__ __forceinline__ void pack_block(const PackOperand& o, long long block) {
+__device__ __forceinline__ void pack_block(const PackOperand& o, unsigned block) {
   const int per_row = o.dcols / 8;
-  const long long v = block * 256 + threadIdx.x;
+  const int matrix = (int)(block / o.blocks);
+  const long long v = (long long)(block % o.blocks) * 256 + threadIdx.x;
   const long long r = v / per_row;
   if (r >= o.drows) return;
   const int c = (int)(v - r * per_row) * 8;
-  const T* s = reinterpret_cast<const T*>(o.src) + r * o.ld + c;
+  const T* s = reinterpret_cast<const T*>(o.src) + matrix % o.batch_inner * o.si + matrix / o.batch_inner * o.so +
+               r * o.ld + c;
   float x[8];
   const int left = r < o.rows ? o.cols - c : 0;
   if (left >= 8) {
@@ -487,7 +491,7 @@ __device__ __forceinline__ void pack_block(const PackOperand& o, long long block
 #pragma unroll
     for (int i = 0; i < 8; ++i) x[i] = i < left ? VecIO<T>::ld(s + i) : 0.0f;
   }
-  __nv_bfloat16* d = o.dst + r * o.dst_ld + c;
+  __nv_bfloat16* d = o.dst + matrix * o.dst_matrix + r * o.dst_ld + c;
   VecIO<__nv_bfloat16>::store(d, x);
   if (sizeof(T) == 4) {
 #pragma unroll
@@ -497,55 +501,69 @@ __device__ __forceinline__ void pack_block(const PackOperand& o, long long block
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) pack_kernel(const PackOperand a, const PackOperand b, const int a_blocks) {
+__global__ void __launch_bounds__(256) pack_kernel(const PackOperand a, const PackOperand b, const unsigned a_blocks) {
   pdl_enter();
-  if ((int)blockIdx.x < a_blocks) pack_block<T>(a, blockIdx.x);
-  else pack_block<T>(b, (long long)blockIdx.x - a_blocks);
+  if (blockIdx.x < a_blocks) pack_block<T>(a, blockIdx.x);
+  else pack_block<T>(b, blockIdx.x - a_blocks);
 }
 
 long long round_up(long long v, long long q) { return (v + q - 1) / q * q; }
 
-PackOperand pack_operand(const void* src, int64_t ld, int mn_major, int outer, int K, int parts) {
+long long batch_of(const GemmArgs& a) {
+  return (long long)(a.batch_inner < 1 ? 1 : a.batch_inner) * (a.batch_outer < 1 ? 1 : a.batch_outer);
+}
+
+PackOperand pack_operand(const GemmArgs& g, bool is_a) {
+  const int parts = g.ab_fp32 ? 2 : 1, Kp = (int)round_up(g.K, 64);
+  const int outer = is_a ? g.M : g.N;
   PackOperand o;
-  const int Kp = (int)round_up(K, 128);
-  o.src = src; o.dst = nullptr; o.ld = ld;
-  if (mn_major) {
-    o.rows = K; o.cols = outer; o.drows = Kp; o.dcols = (int)round_up(outer, 8);
+  o.src = is_a ? g.A : g.B; o.dst = nullptr; o.ld = is_a ? g.lda : g.ldb;
+  o.si = is_a ? g.a_stride_inner : g.b_stride_inner;
+  o.so = is_a ? g.a_stride_outer : g.b_stride_outer;
+  o.batch_inner = g.batch_inner < 1 ? 1 : g.batch_inner;
+  if (is_a ? g.a_mn_major : g.b_mn_major) {
+    o.rows = g.K; o.cols = outer; o.drows = Kp; o.dcols = (int)round_up(outer, 8);
     o.dst_ld = o.dcols;
     o.lo = (long long)Kp * o.dst_ld;
   } else {
-    o.rows = outer; o.cols = K; o.drows = outer; o.dcols = Kp;
+    o.rows = outer; o.cols = g.K; o.drows = outer; o.dcols = Kp;
     o.dst_ld = (long long)parts * Kp;
     o.lo = Kp;
   }
+  o.dst_matrix = (long long)parts * o.drows * o.dcols;
+  o.blocks = (int)(((long long)o.drows * (o.dcols / 8) + 255) / 256);
   return o;
 }
-size_t pack_bytes(const PackOperand& o, int parts) { return (size_t)round_up((long long)parts * o.drows * o.dcols * 2, 256); }
-int pack_blocks(const PackOperand& o) { return (int)(((long long)o.drows * (o.dcols / 8) + 255) / 256); }
+size_t pack_bytes(const PackOperand& o, long long batch) { return (size_t)round_up(batch * o.dst_matrix * 2, 256); }
 
 }  // namespace
 
 size_t gemm_pack_bytes(const GemmArgs& a) {
-  const int parts = a.ab_fp32 ? 2 : 1;
-  return pack_bytes(pack_operand(a.A, a.lda, a.a_mn_major, a.M, a.K, parts), parts) +
-         pack_bytes(pack_operand(a.B, a.ldb, a.b_mn_major, a.N, a.K, parts), parts);
+  return pack_bytes(pack_operand(a, true), batch_of(a)) + pack_bytes(pack_operand(a, false), batch_of(a));
+}
+
+bool gemm_pack_fits(const GemmArgs& a) {
+  const long long batch = batch_of(a);
+  return batch * (pack_operand(a, true).blocks + (long long)pack_operand(a, false).blocks) < (1ll << 31);
 }
 
 cudaError_t gemm_pack(GemmArgs& g, void* workspace, cudaStream_t stream) {
   const int parts = g.ab_fp32 ? 2 : 1;
-  PackOperand a = pack_operand(g.A, g.lda, g.a_mn_major, g.M, g.K, parts);
-  PackOperand b = pack_operand(g.B, g.ldb, g.b_mn_major, g.N, g.K, parts);
+  const long long batch = batch_of(g);
+  PackOperand a = pack_operand(g, true), b = pack_operand(g, false);
   a.dst = (__nv_bfloat16*)workspace;
-  b.dst = (__nv_bfloat16*)((char*)workspace + pack_bytes(a, parts));
-  const int na = pack_blocks(a), nb = pack_blocks(b);
+  b.dst = (__nv_bfloat16*)((char*)workspace + pack_bytes(a, batch));
+  const unsigned na = (unsigned)(a.blocks * batch), nb = (unsigned)(b.blocks * batch);
   const cudaError_t e = g.ab_fp32
       ? launch_pdl(pack_kernel<float>, dim3(na + nb), dim3(256), 0, stream, a, b, na)
       : launch_pdl(pack_kernel<__nv_bfloat16>, dim3(na + nb), dim3(256), 0, stream, a, b, na);
   if (e != cudaSuccess) return e;
   g_gemm_launches.fetch_add(1, std::memory_order_relaxed);
-  const int Kp = (int)round_up(g.K, 128);
+  const int Kp = (int)round_up(g.K, 64);
   g.A = a.dst; g.lda = a.dst_ld;
   g.B = b.dst; g.ldb = b.dst_ld;
+  g.a_stride_inner = a.dst_matrix; g.a_stride_outer = a.dst_matrix * a.batch_inner;
+  g.b_stride_inner = b.dst_matrix; g.b_stride_outer = b.dst_matrix * b.batch_inner;
   if (parts == 2) { g.k_seg = Kp; g.K = 3 * Kp; }
   g.ab_fp32 = 0;
   return cudaSuccess;

@@ -12,6 +12,7 @@ double gemm_direct_cost(const GemmArgs& a);
 // Packing operands for the TMA kernels: bytes of workspace, and the launch that fills it and
 // rewrites `a` to the packed product.
 size_t gemm_pack_bytes(const GemmArgs& a);
+bool gemm_pack_fits(const GemmArgs& a);   // one launch holds all of its blocks
 cudaError_t gemm_pack(GemmArgs& a, void* workspace, cudaStream_t stream);
 // Error word of its bounded waits (0 = ok).  Reading synchronises.
 int gemm_direct_last_error();

@@ -81,11 +81,12 @@ struct TileCfg {
 
 __device__ int g_gemm_error = 0;
 
-// The k blocks of A (in: the block of the product) and B for hi*hi, hi*lo, lo*hi (GemmArgs::k_seg).
+// The k blocks of A (in: the block of the product) and B for hi*hi, hi*lo, lo*hi (GemmArgs::k_seg).  A
+// pipeline stage may reach one block past the end: both are then out of range and load zeros.
 __device__ __forceinline__ void hi_lo_blocks(int seg, int& kA, int& kB) {
   const int part = kA / seg, k = kA - part * seg;
-  kA = part == 2 ? seg + k : k;
-  kB = part == 1 ? seg + k : k;
+  kA = part == 3 ? 2 * seg : part == 2 ? seg + k : k;
+  kB = part == 3 ? 2 * seg : part == 1 ? seg + k : k;
 }
 
 __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
@@ -1531,15 +1532,15 @@ bool gemm_debug() {
 // grows by half a microsecond per 32 values).  Packing costs a launch and a pass over the
 // operands, then runs at TMA speed; the direct kernel reads fp32 through L1 for every tile.
 // Measured: fp32 [1021,777] x [777,1333] 22.9 us packed, 27.3 direct; [1000,1000]^2 22.9 and 19.8;
-// [4096,4096]^2 343 and 558.  The tile model is fitted to launches that follow an idle stream and
+// [4096,4096]^2 343 and 558, two of them 607 and 1078; 96 x [1000,64] x [64,1000] 123 and 483.  The tile model is fitted to launches that follow an idle stream and
 // overestimates the packed product, whose prologue overlaps the packing, by about a quarter.
 Route choose_route(const GemmArgs& a, bool have_workspace) {
   const long long batch = (long long)(a.batch_inner < 1 ? 1 : a.batch_inner) * (a.batch_outer < 1 ? 1 : a.batch_outer);
   if ((long long)a.M * a.N * a.K <= 1 << 17) return ROUTE_SIMT;
-  if (!have_workspace || batch > 1 || a.causal_tiles) return ROUTE_DIRECT;
-  const double elems = (double)a.M * a.K + (double)a.K * a.N;
+  if (!have_workspace || a.causal_tiles || !gemm_pack_fits(a)) return ROUTE_DIRECT;
+  const double elems = (double)batch * ((double)a.M * a.K + (double)a.K * a.N);
   const int parts = a.ab_fp32 ? 3 : 1;
-  const double pack = 0.8 * (3.5e-6 + elems * 8.0 / 4.0e12 + choose_tile(a, parts * a.K, 1, a.c_fp32 != 0).cost);
+  const double pack = 0.8 * (3.5e-6 + elems * 8.0 / 4.0e12 + choose_tile(a, parts * a.K, batch, a.c_fp32 != 0).cost);
   const double direct = gemm_direct_cost(a);
   if (gemm_debug())
     fprintf(stderr, "gemm %dx%dx%d: packed %.1f us, direct %.1f us\n", a.M, a.N, a.K, pack * 1e6, direct * 1e6);
@@ -1589,7 +1590,8 @@ cudaError_t gemm_bf16(const GemmArgs& args, cudaStream_t stream) {
     const cudaError_t e = gemm_pack(a, a.workspace, stream);
     if (e != cudaSuccess) return e;
     a.workspace = nullptr;
-    return launch_choice(choose_tile(a, a.K, 1, a.c_fp32 != 0), a, stream);
+    const long long batch = (long long)(a.batch_inner < 1 ? 1 : a.batch_inner) * (a.batch_outer < 1 ? 1 : a.batch_outer);
+    return launch_choice(choose_tile(a, a.K, batch, a.c_fp32 != 0), a, stream);
   }
   TileChoice tile;
   int splits = choose_split(a, &tile);

@@ -79,3 +79,34 @@ def test_more_matrices_than_a_grid_dimension_holds(M, N, K, dtype):
     for i in (0, 1, 32767, 65535, 65536, n - 1):
         _check(out[i], a[i], b[i], dtype)
     assert _C.gemm_device_error() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("a_t,b_t", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("M,N,K,packed", [(1030, 777, 1001, True), (2047, 1029, 150, True), (64, 24, 700, False)])
+def test_batches_in_two_levels(M, N, K, packed, a_t, b_t, dtype):
+    """Four matrices as 2 x 2 with gaps between them, on the packed and the direct route."""
+    import luatorch_b200 as lf
+    from luatorch_b200 import _C
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+
+    def mats(rows, cols):       # odd rows, a gap behind each matrix and another behind each pair
+        ld, inner = cols + 1, rows * (cols + 1) + 3
+        outer = 2 * inner + 5
+        return torch.randn(2 * outer, generator=g, device="cuda").to(dtype), ld, inner, outer
+
+    def matrix(t, i, o, rows, cols, ld, inner, outer):
+        return t[o * outer + i * inner:][:rows * ld].view(rows, ld)[:, :cols]
+
+    sa, sb = ((K, M) if a_t else (M, K)), ((N, K) if b_t else (K, N))
+    a, b = mats(*sa), mats(*sb)
+    out = torch.zeros(2, 2, M, N, device="cuda", dtype=dtype)
+    before = sum(lf.launch_counts())
+    _C.gemm(a[0], b[0], out, M, N, K, a[1], b[1], N, a_t, not b_t, 2, 2, a[2], a[3], b[2], b[3], M * N, 2 * M * N,
+            1.0, False, None, 0, None, 0, None, None, 0, 0)
+    assert sum(lf.launch_counts()) - before == (2 if packed else 1)
+    for o in range(2):
+        for i in range(2):
+            x, y = matrix(a[0], i, o, *sa, *a[1:]), matrix(b[0], i, o, *sb, *b[1:])
+            _check(out[o, i], x.t() if a_t else x, y.t() if b_t else y, dtype)
+    assert _C.gemm_device_error() == 0
