@@ -971,8 +971,10 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
 // ------------------------------------------------------------------------------
 // SIMT kernel: bf16 or fp32 operands of any stride and alignment, fp32 arithmetic, same
-// epilogue.  For products of a few thousand multiplications (the XOR network's), where filling
-// a 128-row tensor-core tile and draining it takes longer than the sums.
+// epilogue.  For products of a few k steps (the XOR network's, a classifier head's gradients), where
+// filling a 128-row tensor-core tile and draining it takes longer than the sums, see choose_route().
+// A step of 32 values of k is bound by shared-memory reads, two 8-byte ones per four FMAs, and takes
+// 0.95 us (1.75 with four 4-byte reads and without the next step's values on their way).
 // ------------------------------------------------------------------------------
 __device__ __forceinline__ float to_f32(float v) { return v; }
 __device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
@@ -984,8 +986,8 @@ gemm_simt_kernel(const E* __restrict__ A, const E* __restrict__ B,
                  long long a_stride_inner, long long a_stride_outer, long long b_stride_inner,
                  long long b_stride_outer, KernelParams p) {
   constexpr int T = 32, KT = 32;
-  __shared__ float sa[KT][T + 1];
-  __shared__ float sb[KT][T + 1];
+  __shared__ __align__(8) float sa[2][KT][T + 2];
+  __shared__ __align__(8) float sb[2][KT][T + 2];
   // one grid dimension for tiles and batch: the others end at 65535
   const int tiles = p.tiles_m * p.tiles_n, b = (int)(blockIdx.x / tiles), tile = (int)(blockIdx.x % tiles);
   const int bi = b % p.batch_inner, bo = b / p.batch_inner;
@@ -996,33 +998,43 @@ gemm_simt_kernel(const E* __restrict__ A, const E* __restrict__ B,
   const int m0 = tile / p.tiles_n * T, n0 = tile % p.tiles_n * T;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // 16 x 16 threads, 2x2 outputs each
   float acc[2][2] = {{0, 0}, {0, 0}};
-  for (int k0 = 0; k0 < p.K; k0 += KT) {
-    for (int i = threadIdx.x; i < T * KT; i += 256) {
-      int kk, mm;
-      if (a_sk == 1) { kk = i % KT; mm = i / KT; } else { mm = i % T; kk = i / T; }
-      int m = m0 + mm, k = k0 + kk;
-      sa[kk][mm] = (m < p.M && k < p.K) ? to_f32(A[m * a_sm + k * a_sk]) : 0.0f;
-      int nn;
-      if (b_sk == 1) { kk = i % KT; nn = i / KT; } else { nn = i % T; kk = i / T; }
-      int n = n0 + nn;
-      k = k0 + kk;
-      sb[kk][nn] = (n < p.N && k < p.K) ? to_f32(B[k * b_sk + n * b_sn]) : 0.0f;
+  // this thread's four values of each operand per step: neighbouring threads along the contiguous index
+  constexpr int R = T * KT / 256;
+  const bool a_k = a_sk == 1, b_k = b_sk == 1;
+  E ra[R], rb[R];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int i = threadIdx.x + 256 * r, lo = i % 32, hi = i / 32;
+      const int m = m0 + (a_k ? hi : lo), ka = k0 + (a_k ? lo : hi);
+      ra[r] = m < p.M && ka < p.K ? A[m * a_sm + ka * a_sk] : E(0.0f);
+      const int n = n0 + (b_k ? hi : lo), kb = k0 + (b_k ? lo : hi);
+      rb[r] = n < p.N && kb < p.K ? B[kb * b_sk + n * b_sn] : E(0.0f);
     }
-    __syncthreads();
-#pragma unroll 8
+  };
+  load(0);
+  for (int k0 = 0, buf = 0; k0 < p.K; k0 += KT, buf ^= 1) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int i = threadIdx.x + 256 * r, lo = i % 32, hi = i / 32;
+      sa[buf][a_k ? lo : hi][a_k ? hi : lo] = to_f32(ra[r]);
+      sb[buf][b_k ? lo : hi][b_k ? hi : lo] = to_f32(rb[r]);
+    }
+    __syncthreads();                      // the other buffer has been read by everyone who got here
+    if (k0 + KT < p.K) load(k0 + KT);     // the next step's values arrive under this one's sums
+#pragma unroll
     for (int kk = 0; kk < KT; ++kk) {
-      float a0 = sa[kk][ty], a1 = sa[kk][ty + 16];
-      float b0 = sb[kk][tx], b1 = sb[kk][tx + 16];
-      acc[0][0] += a0 * b0; acc[0][1] += a0 * b1;
-      acc[1][0] += a1 * b0; acc[1][1] += a1 * b1;
+      const float2 a = *reinterpret_cast<const float2*>(&sa[buf][kk][2 * ty]);
+      const float2 b = *reinterpret_cast<const float2*>(&sb[buf][kk][2 * tx]);
+      acc[0][0] += a.x * b.x; acc[0][1] += a.x * b.y;
+      acc[1][0] += a.y * b.x; acc[1][1] += a.y * b.y;
     }
-    __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      int m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
+      int m = m0 + 2 * ty + i, n = n0 + 2 * tx + j;
       if (m < p.M && n < p.N) epilogue_store_scalar(p, c_base, m, n, acc[i][j]);
     }
 }
@@ -1528,15 +1540,17 @@ bool gemm_debug() {
   return on;
 }
 
-// SIMT up to 2^17 multiplications (5.4 us either way at 64 x 64 x 64; beyond, its serial k loop
-// grows by half a microsecond per 32 values).  Packing costs a launch and a pass over the
+// SIMT up to four of its k steps and 1024 tile steps, where it is the fastest or loses 1.5 us at most
+// (8 x 8 x 128: 5.8 us, 4.7 direct; 1000 x 1000 x 32: 8.6 and 7.7; 8 x 8 x 2048: 63 and 7.3), and its
+// sums are fp32 FMAs of the whole operands in the order of k.  Packing costs a launch and a pass over the
 // operands, then runs at TMA speed; the direct kernel reads fp32 through L1 for every tile.
 // Measured: fp32 [1021,777] x [777,1333] 22.9 us packed, 27.3 direct; [1000,1000]^2 22.9 and 19.8;
 // [4096,4096]^2 343 and 558, two of them 607 and 1078; 96 x [1000,64] x [64,1000] 123 and 483.  The tile model is fitted to launches that follow an idle stream and
 // overestimates the packed product, whose prologue overlaps the packing, by about a quarter.
 Route choose_route(const GemmArgs& a, bool have_workspace) {
   const long long batch = (long long)(a.batch_inner < 1 ? 1 : a.batch_inner) * (a.batch_outer < 1 ? 1 : a.batch_outer);
-  if ((long long)a.M * a.N * a.K <= 1 << 17) return ROUTE_SIMT;
+  const long long steps = (a.K + 31) / 32, tiles = (long long)((a.M + 31) / 32) * ((a.N + 31) / 32) * batch;
+  if (steps <= 4 && steps * tiles <= 1024) return ROUTE_SIMT;
   if (!have_workspace || a.causal_tiles || !gemm_pack_fits(a)) return ROUTE_DIRECT;
   const double elems = (double)batch * ((double)a.M * a.K + (double)a.K * a.N);
   const int parts = a.ab_fp32 ? 3 : 1;

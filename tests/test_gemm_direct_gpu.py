@@ -110,3 +110,23 @@ def test_batches_in_two_levels(M, N, K, packed, a_t, b_t, dtype):
             x, y = matrix(a[0], i, o, *sa, *a[1:]), matrix(b[0], i, o, *sb, *b[1:])
             _check(out[o, i], x.t() if a_t else x, y.t() if b_t else y, dtype)
     assert _C.gemm_device_error() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("batch,M,N,K,simt", [
+    (1, 1000, 1000, 32, True), (1, 1000, 1025, 32, False),          # 1024 tile steps and one column more
+    (1, 256, 1024, 128, True), (1, 256, 1024, 129, False),          # four steps of k and one value more
+    (64, 32, 127, 128, True), (65, 32, 127, 128, False),
+])
+def test_border_of_the_simt_kernel(batch, M, N, K, simt, dtype):
+    """One launch of fp32 FMAs up to the border: no part of an fp32 operand is lost there."""
+    from luatorch_b200 import _backend as B
+    g = torch.Generator(device="cuda").manual_seed(N)
+    a, b = torch.randn(batch, M, K, generator=g, device="cuda").to(dtype), torch.randn(batch, K, N + 1, generator=g, device="cuda").to(dtype)
+    b = b[:, :, :N].contiguous()
+    out = B.bmm(a, b)
+    for i in {0, batch - 1}:
+        _check(out[i], a[i], b[i], dtype)
+        if simt and dtype == torch.float32:
+            ad, bd = a[i].double(), b[i].double()
+            assert bool(((out[i].double() - ad @ bd).abs() <= K * 2.0 ** -24 * (ad.abs() @ bd.abs())).all())
