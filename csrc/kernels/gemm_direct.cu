@@ -425,7 +425,14 @@ cudaError_t gemm_direct(const GemmArgs& a, cudaStream_t stream) {
 
 double gemm_direct_cost(const GemmArgs& a) {
   const long long batch = (long long)(a.batch_inner < 1 ? 1 : a.batch_inner) * (a.batch_outer < 1 ? 1 : a.batch_outer);
-  return choose_plan(a, a.ab_fp32 != 0, batch).us * 1e-6;
+  const Plan p = choose_plan(a, a.ab_fp32 != 0, batch);
+  const long long tiles = (long long)((a.M + BM - 1) / BM) * ((a.N + p.bn - 1) / p.bn) * batch * p.splits;
+  const double waves = (double)((tiles + sms() - 1) / sms()), rows = (a.M < BM ? a.M : BM) / (double)BM;
+  const double steps = ((a.K + BK - 1) / BK + p.splits - 1) / p.splits;
+  // the plan's own estimate leaves out what the element-wise epilogue takes for its rows; fitted to the
+  // same 455 products as the other routes (choose_route)
+  const double epilogue = (p.bn == 64 ? 3.5 : 7.2) * rows / p.splits + (p.splits > 1 ? 2.1 : 0.0);
+  return 1e-6 * (waves * (0.85 * steps * step_us(p.bn, a.ab_fp32 != 0, a_paired(a) && b_paired(a)) + epilogue + 3.1) - 0.5);
 }
 
 // ------------------------------------------------------------------------------ packing

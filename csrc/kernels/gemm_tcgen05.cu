@@ -1540,24 +1540,53 @@ bool gemm_debug() {
   return on;
 }
 
-// SIMT up to four of its k steps and 1024 tile steps, where it is the fastest or loses 1.5 us at most
-// (8 x 8 x 128: 5.8 us, 4.7 direct; 1000 x 1000 x 32: 8.6 and 7.7; 8 x 8 x 2048: 63 and 7.3), and its
-// sums are fp32 FMAs of the whole operands in the order of k.  Packing costs a launch and a pass over the
-// operands, then runs at TMA speed; the direct kernel reads fp32 through L1 for every tile.
-// Measured: fp32 [1021,777] x [777,1333] 22.9 us packed, 27.3 direct; [1000,1000]^2 22.9 and 19.8;
-// [4096,4096]^2 343 and 558, two of them 607 and 1078; 96 x [1000,64] x [64,1000] 123 and 483.  The tile model is fitted to launches that follow an idle stream and
-// overestimates the packed product, whose prologue overlaps the packing, by about a quarter.
+// Time of the SIMT kernel: 0.95 us per step of its k loop however few outputs there are; beyond one
+// 32 x 32 tile per SM the tiles add to that.
+double simt_cost(const GemmArgs& a, long long batch) {
+  const double tiles = (double)((a.M + 31) / 32) * ((a.N + 31) / 32) * (double)batch;
+  const double steps = (a.K + 31) / 32, more = tiles > 148 ? tiles - 148 : 0.0;
+  return 1e-6 * (2.1 + 0.95 * steps + (0.0034 * steps + 0.0027) * more);
+}
+// Time of the packed product: the pass over the operands, the TMA kernel that follows without a gap,
+// and the element-wise stores of a last column chunk that is not 32 wide.
+double pack_cost(const GemmArgs& a, long long batch) {
+  const long long Kp = (a.K + BK - 1) / BK * BK;
+  const TileChoice t = choose_tile(a, (int)(a.ab_fp32 ? 3 * Kp : Kp), batch, a.c_fp32 != 0);
+  const double bytes = (double)batch * ((double)a.M + a.N) * a.K * (a.ab_fp32 ? 8.0 : 4.0);
+  double edge = 0.0;
+  if (a.N % 32 != 0 && a.ldc % (a.c_fp32 ? 4 : 8) == 0) {
+    const long long tiles = ((a.M + (t.pair ? 2 : 1) * BM - 1) / ((t.pair ? 2 : 1) * BM)) * batch;
+    const long long units = t.pair ? num_sms() / 2 : num_sms();
+    edge = 3.0e-6 * (a.N <= t.bn ? (double)((tiles + units - 1) / units) : 1.0);
+  }
+  return 0.9e-6 + 0.8 * t.cost + bytes / 5.0e12 + edge;
+}
+
+// SIMT up to four of its k steps and 1024 tile steps, where it is the fastest or loses 1.7 us at most
+// (8 x 8 x 128), and its sums are fp32 FMAs of the whole operands in the order of k.  Beyond, the
+// cheapest of the three, by models fitted to each kernel over 455 products (1 to 4096 matrices, M and N
+// from 1 to 8192, K from 1 to 20001, fp32 and bf16, back to back on one stream): the route taken is
+// 1.6 % slower than the best of the three on average, and at worst 1.4 times (5.8 us instead of 4.1).
+//   fp32, us                     SIMT   direct   packed
+//   8 x 8 x 128                   5.9      4.7      8.5
+//   8 x 8 x 2048                 63        7.3     29
+//   300 x 300 x 64                4.3      7.3      9.4
+//   [1000,1000]^2               123       19.8     22.9
+//   [2049,777] x [777,2047]               49.8     26.3
+//   [4095,4095]^2                        570      325
+//   2 x [4096,4096]^2                   1093      634
+//   96 x [1000,64] x [64,1000]  906      483      123
+//   4096 x [32,32]^2             27.7    133       64
 Route choose_route(const GemmArgs& a, bool have_workspace) {
   const long long batch = (long long)(a.batch_inner < 1 ? 1 : a.batch_inner) * (a.batch_outer < 1 ? 1 : a.batch_outer);
   const long long steps = (a.K + 31) / 32, tiles = (long long)((a.M + 31) / 32) * ((a.N + 31) / 32) * batch;
   if (steps <= 4 && steps * tiles <= 1024) return ROUTE_SIMT;
-  if (!have_workspace || a.causal_tiles || !gemm_pack_fits(a)) return ROUTE_DIRECT;
-  const double elems = (double)batch * ((double)a.M * a.K + (double)a.K * a.N);
-  const int parts = a.ab_fp32 ? 3 : 1;
-  const double pack = 0.8 * (3.5e-6 + elems * 8.0 / 4.0e12 + choose_tile(a, parts * a.K, batch, a.c_fp32 != 0).cost);
-  const double direct = gemm_direct_cost(a);
+  const double simt = simt_cost(a, batch), direct = gemm_direct_cost(a);
+  const double pack = have_workspace && !a.causal_tiles && gemm_pack_fits(a) ? pack_cost(a, batch) : 1e30;
   if (gemm_debug())
-    fprintf(stderr, "gemm %dx%dx%d: packed %.1f us, direct %.1f us\n", a.M, a.N, a.K, pack * 1e6, direct * 1e6);
+    fprintf(stderr, "gemm %lld x %dx%dx%d: SIMT %.1f us, direct %.1f us, packed %.1f us\n", batch, a.M, a.N, a.K,
+            simt * 1e6, direct * 1e6, pack * 1e6);
+  if (simt < direct && simt < pack) return ROUTE_SIMT;
   return pack < direct ? ROUTE_PACK : ROUTE_DIRECT;
 }
 

@@ -130,3 +130,41 @@ def test_border_of_the_simt_kernel(batch, M, N, K, simt, dtype):
         if simt and dtype == torch.float32:
             ad, bd = a[i].double(), b[i].double()
             assert bool(((out[i].double() - ad @ bd).abs() <= K * 2.0 ** -24 * (ad.abs() @ bd.abs())).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("M,N,K", [(40, 33, 50), (61, 24, 700), (1030, 777, 1001)])     # SIMT, direct, packed
+@pytest.mark.parametrize("what", ["gelu", "dgelu", "relu", "drelu", "residual"])
+def test_fused_epilogues_on_every_route(M, N, K, what, dtype):
+    """bf16 results.  Beside the product's bound: one rounding of the result (2^-8 of it) and of the
+    intermediate written to aux_out, and tanh.approx (2^-11) through gelu (|z| / 2 of it) and gelu'."""
+    from luatorch_b200 import _backend as B
+    g = torch.Generator(device="cuda").manual_seed(K)
+    a, b = (torch.randn(r, c + 1, generator=g, device="cuda").to(dtype)[:, :c] for r, c in ((M, K), (K, N)))
+    a = a * (K ** -0.5)
+    x = torch.randn(M, N, generator=g, device="cuda").bfloat16()
+    bias = torch.randn(N, generator=g, device="cuda")
+    kw = {"gelu": dict(act=1, bias=bias), "dgelu": dict(act=2, aux_in=x), "relu": dict(act=3, bias=bias),
+          "drelu": dict(act=4, aux_in=x), "residual": dict(residual=x, bias=bias)}[what]
+    pre = torch.empty(M, N, device="cuda", dtype=torch.bfloat16) if what in ("gelu", "relu") else None
+    out = B.gemm(a, b, out_dtype=torch.bfloat16, aux_out=pre, **kw).double()
+    z, mag = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+    if what in ("gelu", "relu", "residual"):
+        z = z + bias.double()
+        mag = mag + bias.double().abs()
+    err = mag * (2.0 ** -16 + 3 * K * 2.0 ** -24)
+    xd, c0, c1 = x.double(), 0.7978845608, 0.044715
+    if what == "gelu":
+        ref = torch.nn.functional.gelu(z, approximate="tanh")
+        err = 1.2 * err + 0.5 * z.abs() * 2.0 ** -11
+    elif what == "dgelu":
+        t = torch.tanh(c0 * (xd + c1 * xd ** 3))
+        ref = z * (0.5 * (1 + t) + 0.5 * xd * (1 - t * t) * c0 * (1 + 3 * c1 * xd * xd))
+        err = 1.2 * err + z.abs() * 2.0 ** -11 * (0.5 + xd.abs() * c0 * (1 + 3 * c1 * xd * xd))
+    elif what == "residual":
+        ref = z + xd
+    else:
+        ref = z.clamp(min=0) if what == "relu" else torch.where(xd > 0, z, torch.zeros_like(z))
+    assert bool(((out - ref).abs() <= err + 2.0 ** -8 * ref.abs() + 1e-6).all()), float((out - ref).abs().max())
+    if pre is not None:
+        assert bool(((pre.double() - z).abs() <= mag * (2.0 ** -16 + 3 * K * 2.0 ** -24) + 2.0 ** -8 * z.abs() + 1e-6).all())
