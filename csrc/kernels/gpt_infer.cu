@@ -27,6 +27,8 @@
 #include "ops.h"
 #include "sm100_ptx.cuh"
 
+#include <algorithm>
+
 namespace lt {
 namespace {
 
@@ -787,7 +789,37 @@ Split choose_split(int N, int K, int G, int max_ks) {
 
 int64_t up(int64_t v) { return (v + 255) & ~int64_t(255); }
 
-struct FwdBuffers { char *x, *n, *qkv, *att, *h; float* stats; };
+// A dense layer's product as the layer classes issue it: [M, K] x [K, N] (+ bias, activation, residual).
+GemmArgs dense_args(const void* a, int64_t lda, const void* W, int64_t ldw, const void* bias, int act,
+                    const void* residual, void* out, int64_t ldo, int64_t M, int N, int K) {
+  GemmArgs g;
+  g.M = (int)M; g.N = N; g.K = K;
+  g.A = a; g.lda = lda; g.B = W; g.ldb = ldw; g.C = out; g.ldc = ldo;
+  g.bias = bias; g.act = act;
+  g.residual = residual; g.ldr = ldo;
+  return g;
+}
+
+// Scratch that the products of a forward over T tokens use (split-K, packed weights), so that they take
+// the same route as in the layers.  The activations' buffers are aligned; a layer is looked at again
+// where the addresses of its matrices allow less than the first one's.
+size_t dense_workspace(const GptWeights& w, int64_t T) {
+  const int E = w.embed, F = w.ffn;
+  const auto odd = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 != 0; };
+  size_t need = gemm_workspace_bytes(dense_args(nullptr, E, w.head, w.head_ld, nullptr, 0, nullptr, nullptr, w.head_ld, T, w.vocab, E));
+  const auto at_least = [&](const GemmArgs& g) { need = std::max(need, gemm_workspace_bytes(g)); };
+  for (int l = 0; l < w.layers; ++l) {
+    const GptLayer &y = w.layer[l], &z = w.layer[0];
+    const void* x = w.tok;   // stands for a residual: one is added
+    if (l == 0 || odd(y.wqkv) != odd(z.wqkv)) at_least(dense_args(nullptr, E, y.wqkv, 3 * E, nullptr, 0, nullptr, nullptr, 3 * E, T, 3 * E, E));
+    if (l == 0 || odd(y.wo) != odd(z.wo)) at_least(dense_args(nullptr, E, y.wo, E, y.bo, 0, x, nullptr, E, T, E, E));
+    if (l == 0 || odd(y.w1) != odd(z.w1)) at_least(dense_args(nullptr, E, y.w1, F, y.b1, GEMM_ACT_GELU, nullptr, nullptr, F, T, F, E));
+    if (l == 0 || odd(y.w2) != odd(z.w2)) at_least(dense_args(nullptr, F, y.w2, E, y.b2, 0, x, nullptr, E, T, E, F));
+  }
+  return need;
+}
+
+struct FwdBuffers { char *x, *n, *qkv, *att, *h; float* stats; char* gemm; size_t gemm_bytes; };
 FwdBuffers carve(const GptWeights& w, int64_t T, void* ws) {
   char* p = (char*)ws;
   FwdBuffers b;
@@ -796,24 +828,22 @@ FwdBuffers carve(const GptWeights& w, int64_t T, void* ws) {
   b.qkv = p; p += up(T * w.embed * 6);
   b.att = p; p += up(T * w.embed * 2);
   b.h = p; p += up(T * w.ffn * 2);
-  b.stats = (float*)p;
+  b.stats = (float*)p; p += up(T * 8);
+  b.gemm = p;
+  b.gemm_bytes = dense_workspace(w, T);
   return b;
 }
 
-cudaError_t dense(const void* a, int64_t lda, const void* W, int64_t ldw, const void* bias, int act,
-                  const void* residual, void* out, int64_t ldo, int64_t M, int N, int K, cudaStream_t s) {
-  GemmArgs g;
-  g.M = (int)M; g.N = N; g.K = K;
-  g.A = a; g.lda = lda; g.B = W; g.ldb = ldw; g.C = out; g.ldc = ldo;
-  g.bias = bias; g.act = act;
-  g.residual = residual; g.ldr = ldo;
+cudaError_t dense(const FwdBuffers& b, GemmArgs g, cudaStream_t s) {
+  g.workspace = b.gemm_bytes ? b.gemm : nullptr;
+  g.workspace_bytes = b.gemm_bytes;
   return gemm_bf16(g, s);
 }
 
 }  // namespace
 
 size_t gpt_forward_workspace(const GptWeights& w, int64_t T) {
-  return (size_t)(up(T * w.embed * 2) * 3 + up(T * w.embed * 6) + up(T * w.ffn * 2) + up(T * 8));
+  return (size_t)(up(T * w.embed * 2) * 3 + up(T * w.embed * 6) + up(T * w.ffn * 2) + up(T * 8)) + dense_workspace(w, T);
 }
 
 cudaError_t gpt_forward(const GptWeights& w, const void* ids, int id_kind, int64_t batch, int64_t seq,
@@ -828,7 +858,7 @@ cudaError_t gpt_forward(const GptWeights& w, const void* ids, int id_kind, int64
     const GptLayer& y = w.layer[l];
     char* qkv = cache ? (char*)cache + (int64_t)l * cache_rows * E * 6 : b.qkv;
     e = layernorm_forward(DT_BF16, b.x, y.ln1_g, y.ln1_b, DT_BF16, w.eps, b.n, mean, rstd, T, E, s);
-    if (e == cudaSuccess) e = dense(b.n, E, y.wqkv, 3 * E, nullptr, 0, nullptr, qkv, 3 * E, T, 3 * E, E, s);
+    if (e == cudaSuccess) e = dense(b, dense_args(b.n, E, y.wqkv, 3 * E, nullptr, 0, nullptr, qkv, 3 * E, T, 3 * E, E), s);
     AttnArgs a;
     a.B = (int)batch; a.H = w.heads; a.S = (int)seq; a.D = w.head_dim;
     a.q = qkv; a.k = qkv + 2 * E; a.v = qkv + 4 * E; a.o = b.att;
@@ -837,10 +867,10 @@ cudaError_t gpt_forward(const GptWeights& w, const void* ids, int id_kind, int64
     a.o_ss = E; a.o_sb = seq * E;
     a.causal = 1; a.scale = w.scale;
     if (e == cudaSuccess) e = flash_attention_forward(a, s);
-    if (e == cudaSuccess) e = dense(b.att, E, y.wo, E, y.bo, 0, b.x, b.x, E, T, E, E, s);
+    if (e == cudaSuccess) e = dense(b, dense_args(b.att, E, y.wo, E, y.bo, 0, b.x, b.x, E, T, E, E), s);
     if (e == cudaSuccess) e = layernorm_forward(DT_BF16, b.x, y.ln2_g, y.ln2_b, DT_BF16, w.eps, b.n, mean, rstd, T, E, s);
-    if (e == cudaSuccess) e = dense(b.n, E, y.w1, F, y.b1, GEMM_ACT_GELU, nullptr, b.h, F, T, F, E, s);
-    if (e == cudaSuccess) e = dense(b.h, F, y.w2, E, y.b2, 0, b.x, b.x, E, T, E, F, s);
+    if (e == cudaSuccess) e = dense(b, dense_args(b.n, E, y.w1, F, y.b1, GEMM_ACT_GELU, nullptr, b.h, F, T, F, E), s);
+    if (e == cudaSuccess) e = dense(b, dense_args(b.h, F, y.w2, E, y.b2, 0, b.x, b.x, E, T, E, F), s);
   }
   *x_out = b.x;
   return e;
@@ -851,7 +881,7 @@ cudaError_t gpt_logits(const GptWeights& w, const void* x, int64_t n, void* work
   const FwdBuffers b = carve(w, n, workspace);
   cudaError_t e = layernorm_forward(DT_BF16, x, w.lnf_g, w.lnf_b, DT_BF16, w.eps, b.n, b.stats, b.stats + n, n, w.embed, s);
   if (e == cudaSuccess)
-    e = dense(b.n, w.embed, w.head, w.head_ld, nullptr, 0, nullptr, logits, w.head_ld, n, w.vocab, w.embed, s);
+    e = dense(b, dense_args(b.n, w.embed, w.head, w.head_ld, nullptr, 0, nullptr, logits, w.head_ld, n, w.vocab, w.embed), s);
   return e;
 }
 

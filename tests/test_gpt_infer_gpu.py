@@ -350,3 +350,17 @@ def test_decode_draws_the_exact_token(vocab, top_k, embed):
         assert lo - 1e-4 <= r <= float(cdf[t]) + 1e-4, (i, t, lo, r, float(cdf[t]))
         if abs(lo - r) > 1e-4 and abs(float(cdf[t]) - r) > 1e-4:
             assert t == int(torch.searchsorted(cdf, torch.tensor(r, dtype=torch.float64)))
+
+
+@pytest.mark.parametrize("embed,ffn,batch,seq", [(2048, 8192, 1, 64), (2304, 2304, 1, 17), (2048, 8192, 3, 100), (128, 4104, 1, 200)])
+def test_long_products_of_short_prompts_are_the_layers(embed, ffn, batch, seq):
+    """Products that the layers cut along K are cut here too: the same bits."""
+    import luatorch_b200 as lf
+    lf.manual_seed(4)
+    m = lf.models.GPT(97, embed, embed // 128, 1, 128, 0.0, pos="learned")
+    m.blocks[0].ffn1, m.blocks[0].ffn2 = lf.nn.Linear(embed, ffn), lf.nn.Linear(ffn, embed)
+    lf.cuda.amp.autocast_bf16(m)
+    m.eval()
+    assert m._inference_weights() is not None
+    ids = torch.randint(0, 97, (batch, seq), device="cuda", dtype=torch.int32)
+    assert _same_as_layers(m, ids)
