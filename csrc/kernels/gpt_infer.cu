@@ -44,7 +44,8 @@ constexpr long long BARRIER_BUDGET = 4000000000ll;   // about two seconds of SM 
 
 // Where a [K, N] product is cut: `nu` units of 8 columns per CTA, `ks` slices of K.
 struct Split { int nu, groups, ks; };   // nu: power of two, at most 16
-constexpr int MAX_KS = 16;
+constexpr int MAX_KS = 16;           // partial sums per element that a consumer adds (out_head: one per head)
+constexpr int SPLIT_KS = 4;          // of a product cut over K for its own sake
 
 struct DecodeParams {
   GptWeights w;
@@ -52,7 +53,7 @@ struct DecodeParams {
   bf16* cache;                       // [layers, rows, 3 embed]
   long long cache_rows;
   int prompt, first, last;
-  float inv_temp, temperature;
+  float temperature;
   int top_k;
   const float* rnd;
   int* ids_out;
@@ -777,7 +778,7 @@ Split choose_split(int N, int K, int G, int max_ks) {
   Split best{16, (units + 15) / 16, 1};
   double best_cost = 1e30;
   for (int nu = 2; nu <= 16; nu *= 2)          // 16-byte columns would waste half of each sector
-    for (int ks = 1; ks <= max_ks && ks <= 4 && K / ks >= 64; ++ks) {
+    for (int ks = 1; ks <= max_ks && K / ks >= 64; ++ks) {
       const int groups = (units + nu - 1) / nu;
       const int rounds = (groups * ks + G - 1) / G;
       // 16-byte loads of the busiest CTA, a pass's reduction, the consumers' partial sums
@@ -912,12 +913,12 @@ cudaError_t gpt_decode(const GptWeights& w, const void* x, void* cache, int64_t 
   p.x0 = (const bf16*)x;
   p.cache = (bf16*)cache; p.cache_rows = cache_rows;
   p.prompt = prompt; p.first = first; p.last = last;
-  p.temperature = temperature; p.inv_temp = 1.0f / temperature; p.top_k = top_k;
+  p.temperature = temperature; p.top_k = top_k;
   p.rnd = rnd; p.ids_out = ids_out;
   p.qkv = choose_split(3 * w.embed, w.embed, G, 1);
-  p.out = choose_split(w.embed, w.embed, G, MAX_KS);
+  p.out = choose_split(w.embed, w.embed, G, SPLIT_KS);
   p.f1 = choose_split(w.ffn, w.embed, G, 1);
-  p.f2 = choose_split(w.embed, w.ffn, G, MAX_KS);
+  p.f2 = choose_split(w.embed, w.ffn, G, SPLIT_KS);
   p.head = choose_split(w.vocab, w.embed, G, 1);
   // a head per K slice where that fills the grid in one round; 256 keys are 64 KB of a head's rows
   p.out_head = {0, 0, 0};
