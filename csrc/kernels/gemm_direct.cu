@@ -424,7 +424,7 @@ cudaError_t gemm_direct(const GemmArgs& a, cudaStream_t stream) {
 }
 
 double gemm_direct_cost(const GemmArgs& a) {
-  const long long batch = (long long)(a.batch_inner < 1 ? 1 : a.batch_inner) * (a.batch_outer < 1 ? 1 : a.batch_outer);
+  const long long batch = (long long)a.batch_inner * a.batch_outer;
   const Plan p = choose_plan(a, a.ab_fp32 != 0, batch);
   const long long tiles = (long long)((a.M + BM - 1) / BM) * ((a.N + p.bn - 1) / p.bn) * batch * p.splits;
   const double waves = (double)((tiles + sms() - 1) / sms()), rows = (a.M < BM ? a.M : BM) / (double)BM;
@@ -517,7 +517,7 @@ __global__ void __launch_bounds__(256) pack_kernel(const PackOperand a, const Pa
 long long round_up(long long v, long long q) { return (v + q - 1) / q * q; }
 
 long long batch_of(const GemmArgs& a) {
-  return (long long)(a.batch_inner < 1 ? 1 : a.batch_inner) * (a.batch_outer < 1 ? 1 : a.batch_outer);
+  return (long long)a.batch_inner * a.batch_outer;
 }
 
 PackOperand pack_operand(const GemmArgs& g, bool is_a) {
@@ -527,7 +527,7 @@ PackOperand pack_operand(const GemmArgs& g, bool is_a) {
   o.src = is_a ? g.A : g.B; o.dst = nullptr; o.ld = is_a ? g.lda : g.ldb;
   o.si = is_a ? g.a_stride_inner : g.b_stride_inner;
   o.so = is_a ? g.a_stride_outer : g.b_stride_outer;
-  o.batch_inner = g.batch_inner < 1 ? 1 : g.batch_inner;
+  o.batch_inner = g.batch_inner;
   if (is_a ? g.a_mn_major : g.b_mn_major) {
     o.rows = g.K; o.cols = outer; o.drows = Kp; o.dcols = (int)round_up(outer, 8);
     o.dst_ld = o.dcols;

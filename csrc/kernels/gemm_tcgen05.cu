@@ -1370,8 +1370,7 @@ TileChoice choose_tile(const GemmArgs& a, int K, long long batch, bool c_fp32, b
 
 // Split-K factor for `a` (1 = none) and the tile to use for the slices.
 int choose_split(const GemmArgs& a, TileChoice* slice_tile) {
-  const long long batch = (long long)(a.batch_inner < 1 ? 1 : a.batch_inner) *
-                          (a.batch_outer < 1 ? 1 : a.batch_outer);
+  const long long batch = (long long)a.batch_inner * a.batch_outer;
   TileChoice whole = choose_tile(a, a.K, batch, a.c_fp32 != 0);
   *slice_tile = whole;
   if (batch != 1 || a.act != GEMM_ACT_NONE || a.residual || a.aux_out || a.aux_in ||
@@ -1578,7 +1577,7 @@ double pack_cost(const GemmArgs& a, long long batch) {
 //   96 x [1000,64] x [64,1000]  906      483      123
 //   4096 x [32,32]^2             27.7    133       64
 Route choose_route(const GemmArgs& a, bool have_workspace) {
-  const long long batch = (long long)(a.batch_inner < 1 ? 1 : a.batch_inner) * (a.batch_outer < 1 ? 1 : a.batch_outer);
+  const long long batch = (long long)a.batch_inner * a.batch_outer;
   const long long steps = (a.K + 31) / 32, tiles = (long long)((a.M + 31) / 32) * ((a.N + 31) / 32) * batch;
   if (steps <= 4 && steps * tiles <= 1024) return ROUTE_SIMT;
   const double simt = simt_cost(a, batch), direct = gemm_direct_cost(a);
@@ -1593,7 +1592,7 @@ Route choose_route(const GemmArgs& a, bool have_workspace) {
 }  // namespace
 
 size_t gemm_workspace_bytes(const GemmArgs& a) {
-  if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.gather) return 0;
+  if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.batch_inner <= 0 || a.batch_outer <= 0 || a.gather) return 0;
   if (!gemm_uses_tensor_cores(a)) return choose_route(a, true) == ROUTE_PACK ? gemm_pack_bytes(a) : 0;
   TileChoice t;
   const int s = choose_split(a, &t);
@@ -1604,7 +1603,7 @@ size_t gemm_workspace_bytes(const GemmArgs& a) {
 static thread_local bool g_prev_reads_workspace = false;
 
 cudaError_t gemm_bf16(const GemmArgs& args, cudaStream_t stream) {
-  if (args.M <= 0 || args.N <= 0) return cudaSuccess;
+  if (args.M <= 0 || args.N <= 0 || args.batch_inner <= 0 || args.batch_outer <= 0) return cudaSuccess;
   if (args.K <= 0) return cudaErrorInvalidValue;
   GemmArgs a = args;
   if (a.gather && a.gather->world > 1) a.overlap_prev = 0;
@@ -1633,7 +1632,7 @@ cudaError_t gemm_bf16(const GemmArgs& args, cudaStream_t stream) {
     const cudaError_t e = gemm_pack(a, a.workspace, stream);
     if (e != cudaSuccess) return e;
     a.workspace = nullptr;
-    const long long batch = (long long)(a.batch_inner < 1 ? 1 : a.batch_inner) * (a.batch_outer < 1 ? 1 : a.batch_outer);
+    const long long batch = (long long)a.batch_inner * a.batch_outer;
     return launch_choice(choose_tile(a, a.K, batch, a.c_fp32 != 0), a, stream);
   }
   TileChoice tile;

@@ -168,3 +168,12 @@ def test_fused_epilogues_on_every_route(M, N, K, what, dtype):
     assert bool(((out - ref).abs() <= err + 2.0 ** -8 * ref.abs() + 1e-6).all()), float((out - ref).abs().max())
     if pre is not None:
         assert bool(((pre.double() - z).abs() <= mag * (2.0 ** -16 + 3 * K * 2.0 ** -24) + 2.0 ** -8 * z.abs() + 1e-6).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_no_matrices(dtype):
+    """A batch of none has nothing to read."""
+    from luatorch_b200 import _backend as B
+    out = B.bmm(torch.empty(0, 20, 30, device="cuda", dtype=dtype), torch.empty(0, 30, 40, device="cuda", dtype=dtype))
+    assert out.shape == (0, 20, 40) and out.dtype == dtype
+    torch.cuda.synchronize()
