@@ -198,12 +198,12 @@ softmax_short_kernel(const T* in, T* out, int64_t rows, int cols, int64_t ld) {
 #pragma unroll
   for (int i = 0; i < NE; ++i) m = fmaxf(m, v[i]);
   m = warp_max(m);
-  const float c0 = -m * LOG2E;
 #pragma unroll
   for (int i = 0; i < NE; ++i) {
-    // places past the row end hold -inf, which adds nothing unless the whole row is -inf (NaN then,
-    // as the sum of such a row is in any case)
-    v[i] = ex2_fast(fmaf(v[i], LOG2E, c0));
+    // The difference first: m LOG2E alone overflows for a row of the type's lowest values, and loses
+    // the last bits of large ones.  Places past the row end hold -inf, which adds nothing unless the
+    // whole row is -inf (NaN then, as the sum of such a row is in any case).
+    v[i] = ex2_fast((v[i] - m) * LOG2E);
     s += v[i];
   }
   const float r = 1.0f / warp_sum(s);

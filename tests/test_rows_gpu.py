@@ -82,3 +82,25 @@ def test_column_sum_slabs(rows, cols):
     B.column_sum(x, out, True)
     bound = (rows + 1) * 2.0 ** -24 * (xd.abs().sum(0) + 1)
     assert bool(((out.double() - 1 - xd.sum(0)).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("cols", [1, 31, 64, 257, 1000, 1024])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_softmax_of_extreme_rows(cols, dtype):
+    """Rows of the type's lowest value (a mask that leaves nothing) are uniform, as in torch; large
+    values keep the bound, because the difference to the maximum is taken before anything is scaled:
+    arguments down to -87 count, each to 87 2^-23 of its exponential, and the sum to cols 2^-24."""
+    from luatorch_b200 import _backend as B
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    low = torch.finfo(dtype).min
+    x = torch.randn(8, cols, generator=g, device="cuda").to(dtype)
+    x[0] = low
+    x[1, ::2] = low
+    x[2, 1:] = low
+    x[3:6] *= 1000
+    x[6] = torch.finfo(dtype).max
+    y = B.softmax(x).double()
+    ref = torch.softmax(x.double(), 1)
+    lost = {torch.float32: 0.0, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
+    tiny = 2.0 ** -24 if dtype == torch.float16 else 1e-37      # subnormal results
+    assert bool(((y - ref).abs() <= (2e-5 + cols * 2.0 ** -24 + lost) * ref + tiny).all()), float((y - ref).abs().max())
