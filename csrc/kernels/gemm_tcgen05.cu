@@ -1425,7 +1425,8 @@ cudaError_t launch_choice(const TileChoice& t, const GemmArgs& a, cudaStream_t s
 // Bound by latency: a convolution's weight gradient has up to 148 slices of a few thousand elements,
 // and one thread walking all of them took 11.4 us a call (four in the convolution net).  STAGED:
 // eight warps bring 64 slices of the block's 32 quads into shared memory, where each element's
-// chain of sums runs in a thread of its own; the next 64 are on their way meanwhile.
+// chain of sums runs in a thread of its own; the next 64 are on their way meanwhile (32 x 27 over
+// K = 131072 with its product: 58.4 -> 23.6 us).
 template <bool STAGED>
 __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(const float* __restrict__ ws, int splits, long long slice, int M, int N,
